@@ -310,9 +310,10 @@ int mgb_selftest_wait_timeout(void *stream);
  * s to unit 2-norm (normalize! of simple_update); MGB_SVD_CONJ_V writes
  * conj(V), the right factor as tensor_svd_thin labels it; MGB_SVD_SQRT_S
  * writes sqrt of the (normalised) s, for an equal absorb. One-sided Jacobi
- * rotations in one thread block on the device: min(m, n) <= 1024, m n <=
- * 2^28. Left vectors of exactly zero singular values are completed to an
- * orthonormal set. The workspace comes from mgb_svd_workspace_size.        */
+ * rotations on the device, a pair of columns per SM in one cooperative
+ * launch: min(m, n) <= 1024, m n <= 2^28. Left vectors of exactly zero
+ * singular values are completed to an orthonormal set. The workspace comes
+ * from mgb_svd_workspace_size.                                            */
 #define MGB_SVD_NORMALIZE 1
 #define MGB_SVD_CONJ_V 2
 #define MGB_SVD_SQRT_S 4
