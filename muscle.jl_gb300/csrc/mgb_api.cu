@@ -256,7 +256,7 @@ static uint64_t align256(uint64_t x) { return (x + 255) & ~uint64_t(255); }
 // load), so the plain form needs no workspace.
 static void plain_workspace(ContractionPlan &p) {
     p.convert_a = p.convert_b = false;
-    p.ws_bytes = 0;
+    p.ws_bytes = p.ws_min = 0;
 }
 
 }  // namespace mgb
@@ -366,7 +366,7 @@ static int contract_impl(mgb_plan plan, const void *A, const void *B, void *C, v
                          uint64_t workspace_bytes, void *stream) {
     const ContractionPlan &cp = plan->cp;
     cudaStream_t s = (cudaStream_t)stream;
-    if (workspace_bytes < cp.ws_bytes || (cp.ws_bytes && !workspace))
+    if (workspace_bytes < cp.ws_min || (cp.ws_min && !workspace))
         return fail(MGB_ERR_WORKSPACE, "workspace smaller than mgb_plan_workspace_size");
     int64_t nc = cp.M * cp.N * cp.L;
     if (nc == 0) {
@@ -379,7 +379,7 @@ static int contract_impl(mgb_plan plan, const void *A, const void *B, void *C, v
     if (!A || !B) return fail(MGB_ERR_ARGUMENT, "null operand pointer");
     if (cp.swapped) std::swap(A, B);  // the plan computes C^T = B^T A^T
     if (cp.form == MGB_FORM_PLAIN) return launch_plain_gemm(cp, A, B, C, s);
-    return launch_ozaki(cp, A, B, C, workspace, s, plan->timing ? plan->ev[1] : nullptr);
+    return launch_ozaki(cp, A, B, C, workspace, workspace_bytes >= cp.ws_bytes, s, plan->timing ? plan->ev[1] : nullptr);
 }
 
 int mgb_plan_set_timing(mgb_plan plan, int32_t enable) {

@@ -214,7 +214,7 @@ int mgb_group_create(mgb_group *group, const mgb_plan *plans, int32_t count, con
         b.cp.gl.ext[0] = n;
         for (int t = 0; t < 3; ++t) b.cp.gl.str[t][0] = 0;
         if (b.cp.form != MGB_FORM_PLAIN) ozaki_setup(b.cp);  // workspace for L members
-        else b.cp.ws_bytes = 0;
+        else b.cp.ws_bytes = b.cp.ws_min = 0;
         cudaError_t e = cudaMalloc((void **)&b.dptr, 3 * n * sizeof(void *));
         if (e != cudaSuccess) {
             b.dptr = nullptr;
@@ -300,7 +300,7 @@ static int run_unit(mgb_group g, int u, void *workspace, cudaStream_t s) {
     if (u < nb) {
         Bucket &b = g->buckets[u];
         return b.cp.form == MGB_FORM_PLAIN ? launch_plain_gemm(b.cp, nullptr, nullptr, nullptr, s)
-                                           : launch_ozaki(b.cp, nullptr, nullptr, nullptr, (char *)workspace + b.ws_off, s);
+                                           : launch_ozaki(b.cp, nullptr, nullptr, nullptr, (char *)workspace + b.ws_off, true, s);
     }
     const Single &m = g->singles[u - nb];
     const mgb_plan p = g->plans[m.member];
@@ -324,7 +324,7 @@ int mgb_group_prepare_part(mgb_group group, int32_t part, int32_t nparts, void *
     auto one = [&](int u) -> int {
         Bucket &b = group->buckets[u];
         return b.cp.form == MGB_FORM_PLAIN ? launch_plain_gemm(b.cp, nullptr, nullptr, nullptr, s)
-                                           : ozaki_prepass(b.cp, nullptr, nullptr, (char *)workspace + b.ws_off, s);
+                                           : ozaki_prepass(b.cp, nullptr, nullptr, (char *)workspace + b.ws_off, true, s);
     };
     if (nparts == 1) {
         for (int u = 0; u < nb; ++u)

@@ -132,8 +132,16 @@ struct ContractionPlan {
     // exchanged, and every entry point passes the caller's B where the plan
     // says A. Set at plan creation when it fills more of the 128-row tiles.
     bool swapped = false;
-    uint64_t ws_bytes = 0;
+    // Bytes of workspace: what the plan asks for, and what it can run with
+    // (without room for the sums of tiles that are split along K).
+    uint64_t ws_bytes = 0, ws_min = 0;
     // workspace layout (byte offsets)
+    uint64_t ws_cnt = 0, ws_part = 0;  // counters and sums of split tiles
+    // Tiles of the emulated GEMM's last wave are cut along K: the first
+    // `split_full` tiles are whole, the others `splits` units of `split_kbs`
+    // k blocks each (splits = 1: none is cut).
+    int64_t split_full = 0;
+    int32_t splits = 1, split_kbs = 0;
     uint64_t ws_a = 0, ws_b = 0, ws_scale_a = 0, ws_scale_b = 0;
     int64_t kpad = 0;      // padded embedded K of the slice buffers
     int64_t m_e = 0, n_e = 0, k_e = 0;  // embedded GEMM extents
@@ -169,18 +177,20 @@ int launch_fill_zero(void *p, int64_t count, int dtype, const Desc &d, cudaStrea
 // (the adaptive choice "plain").
 int launch_plain_gemm(const ContractionPlan &p, const void *A, const void *B, void *C,
                       cudaStream_t s, const int32_t *sel = nullptr);
+// `split`: the workspace holds ws_bytes, so tiles may be split along K; with
+// ws_min bytes they are not.
 int launch_ozaki(const ContractionPlan &p, const void *A, const void *B, void *C,
-                 void *ws, cudaStream_t s, cudaEvent_t mid = nullptr);
+                 void *ws, bool split, cudaStream_t s, cudaEvent_t mid = nullptr);
 int launch_unary(const UnaryPlan &p, const void *X, void *Y, cudaStream_t s);
 int selftest_wait_timeout(cudaStream_t s);
 // Emulated forms split for groups: the pre-pass of one plan, and one
 // persistent GEMM launch for several plans of one kernel variant (same
 // slices, form and real/complex) whose slices lie in the given workspaces.
-int ozaki_prepass(const ContractionPlan &p, const void *A, const void *B, void *ws, cudaStream_t s);
+int ozaki_prepass(const ContractionPlan &p, const void *A, const void *B, void *ws, bool split, cudaStream_t s);
 // The tensor-core part of one plan whose pre-pass has run into `ws` (for an
 // adaptive plan: one launch per candidate slice count, of which only the
 // chosen one works, and the plain form as the fallback).
-int ozaki_gemm(const ContractionPlan &p, const void *A, const void *B, void *C, void *ws, cudaStream_t s);
+int ozaki_gemm(const ContractionPlan &p, const void *A, const void *B, void *C, void *ws, bool split, cudaStream_t s);
 // Reads the adaptive choice of the last call that ran with `ws` (synchronises s).
 int ozaki_adaptive_report(const ContractionPlan &p, const void *ws, cudaStream_t s, mgb_adaptive_report *out);
 int ozaki_set_tolerance(ContractionPlan &p, double tol);
@@ -199,6 +209,7 @@ struct OzBatchItem {
     const void *A, *B;
     void *C;
     void *ws;
+    bool split;  // `ws` has room for split tiles (ws_bytes, not only ws_min)
 };
 struct OzBatchBuffers;
 OzBatchBuffers *ozaki_batch_buffers_create();

@@ -52,7 +52,7 @@ int scratch_address(void **out) {
 extern "C" int mgb_contract_noalloc(mgb_plan plan, const void *A, const void *B, void *C, void *stream) {
     if (!plan || plan->kind != mgb::PlanKind::Contraction)
         return mgb::fail(MGB_ERR_ARGUMENT, "not a contraction plan");
-    const uint64_t need = plan->cp.ws_bytes;
+    const uint64_t need = plan->cp.ws_min;  // tiles are split along K only where ws_bytes fit
     if (need > (uint64_t)MGB_NOALLOC_SCRATCH_BYTES)
         return mgb::fail(MGB_ERR_WORKSPACE,
                          "contraction needs " + std::to_string(need) +

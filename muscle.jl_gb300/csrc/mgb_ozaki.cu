@@ -817,17 +817,27 @@ __device__ __forceinline__ void oz_slice_tile(const T *__restrict__ X, const OpG
     }
 }
 
+// The first block of an operand's slicing clears the `n` counters of the
+// contraction's split tiles (null for one of its two operands), which the
+// GEMM after it counts with.
+__device__ __forceinline__ void oz_clear_counters(int32_t *cnt, int n) {
+    if (cnt)
+        for (int i = threadIdx.x; i < n; i += blockDim.x) cnt[i] = 0;
+}
+
 // `sel` (nullable): the adaptive choice; the slice count is read from it and
 // the launch does nothing when it is 0 (plain).
 template <typename T, int MODE, bool BF3>
 __global__ void __launch_bounds__(256, 4) k_oz_slice(const T *__restrict__ X, OpGeom g,
                                                   const int32_t *__restrict__ exps, int S,
                                                   uint32_t *__restrict__ out, int64_t rows_e,
-                                                  int64_t kw, const int32_t *__restrict__ sel) {
+                                                  int64_t kw, const int32_t *__restrict__ sel,
+                                                  int32_t *cnt, int ncnt) {
     if (sel) {
         S = *sel;
         if (S == 0) return;
     }
+    if (blockIdx.x == 0 && blockIdx.y == 0) oz_clear_counters(cnt, ncnt);
     __shared__ SliceSmemOf<T, MODE> sm;
     oz_slice_tile<T, MODE, BF3>(X, g, exps, S, out, rows_e, kw, blockIdx.x, blockIdx.y, sm);
 }
@@ -848,6 +858,14 @@ struct OzGemmArgs {
     ModeGroup gm, gn, gl;  // C offsets live in tensor slot 2
     int32_t *status;
     const int32_t *sel;    // adaptive choice (nullable): run only when it holds S
+    // Work units: the first `full` tiles are one unit each, every tile after
+    // them is `splits` units of `kbs` k blocks (see oz_split). A split tile's
+    // units leave their sums in `part` and count in `cnt`; the last one adds
+    // them up and writes the outputs.
+    int32_t splits, kbs;
+    int64_t full;
+    uint32_t *part;
+    int32_t *cnt;
 };
 
 // One contraction (or one bucket of a group) as the GEMM sees it: the slice
@@ -857,17 +875,22 @@ struct OzJob {  // aligned as its tensor maps
     CUtensorMap tmA, tmB;
     OzGemmArgs a;
     int32_t tiles_n, tiles_m, L;
+    __host__ __device__ int64_t units() const {
+        const int64_t t = (int64_t)tiles_n * tiles_m * L;
+        return a.full + (t - a.full) * a.splits;
+    }
 };
 
 // Tile sources of the kernel: one job in the parameter space, or a table of
-// jobs in global memory (a group) whose tiles are numbered consecutively.
-// `hint` is the caller's job index of its previous tile (0 at first): a CTA
-// visits its tiles in increasing order, so the next tile usually lies in the
-// same job or the one after it.
+// jobs in global memory (a group) whose work units (whole tiles, or parts of
+// a split tile) are numbered consecutively. `hint` is the caller's job index
+// of its previous unit (0 at first): a CTA visits its units in increasing
+// order, so the next one usually lies in the same job or the one after it.
 struct OzOneJob {
     static constexpr bool kTable = false;
     const OzJob *j;
-    __device__ int64_t tiles() const { return (int64_t)j->tiles_n * j->tiles_m * j->L; }
+    __device__ int64_t units() const { return j->units(); }
+    __device__ bool any(int) const { return true; }
     __device__ const OzJob &job(int64_t t, int64_t &local, int &) const {
         local = t;
         return *j;
@@ -876,9 +899,14 @@ struct OzOneJob {
 struct OzJobTable {
     static constexpr bool kTable = true;  // jobs may carry their own adaptive choice (skipped unless it is S)
     const OzJob *jobs;
-    const int64_t *start;  // [n + 1]: first tile of each job, then the total
+    const int64_t *start;  // [n + 1]: first unit of each job, then the total
     int n;
-    __device__ int64_t tiles() const { return start[n]; }
+    __device__ int64_t units() const { return start[n]; }
+    __device__ bool any(int S) const {
+        bool mine = false;
+        for (int i = threadIdx.x; i < n; i += blockDim.x) mine = mine || !jobs[i].a.sel || *jobs[i].a.sel == S;
+        return __syncthreads_or(mine);
+    }
     __device__ const OzJob &job(int64_t t, int64_t &local, int &hint) const {
         int lo = hint;  // the last job with start <= t, at or after the hint
         if (lo + 1 < n && start[lo + 1] <= t) {
@@ -939,6 +967,48 @@ __device__ __forceinline__ void oz_tile(const OzJob &J, int64_t local, int bn, i
         oz_tile_t<uint32_t>((uint32_t)local, (uint32_t)nn, (uint32_t)nm, (uint32_t)gm, bn, m0, n0, l);
     else
         oz_tile_t<int64_t>(local, nn, nm, gm, bn, m0, n0, l);
+}
+
+// Work unit `local` of a job: its tile and k blocks [kb0, kb1), and its index
+// among the units of split tiles (-1 for a whole tile). A job's split
+// units are a few waves at most, so their numbers fit 32 bits.
+struct OzUnit {
+    int64_t m0, n0;
+    int l, kb0, kb1, part;
+};
+__device__ __forceinline__ OzUnit oz_unit(const OzJob &J, int64_t local, int bn) {
+    OzUnit u;
+    u.kb0 = 0;
+    u.kb1 = J.a.nkb;
+    u.part = -1;
+    if (local >= J.a.full) {
+        u.part = (int)(local - J.a.full);
+        const int t = u.part / J.a.splits;
+        u.kb0 = (u.part - t * J.a.splits) * J.a.kbs;
+        u.kb1 = min(J.a.nkb, u.kb0 + J.a.kbs);
+        local = J.a.full + t;
+    }
+    oz_tile(J, local, bn, u.m0, u.n0, u.l);
+    return u;
+}
+
+// ---- sums of a split tile ------------------------------------------------------
+// An epilogue warp's share of a unit: NW words per lane, as 16-byte vectors
+// of consecutive lanes.
+template <int NW>
+__device__ __forceinline__ uint4 *oz_part_at(uint32_t *part, int unit, int w) {
+    return (uint4 *)part + (((int64_t)unit * OZ_EPI_WARPS + w) * (NW / 4)) * 32 + threadIdx.x % 32;
+}
+// Publishes this warp's share and counts it; true for the warp that finds all
+// `splits` shares of its tile published. Nobody waits for anybody.
+__device__ __forceinline__ bool oz_part_last(int32_t *cnt, int tile, int w, int splits) {
+    __threadfence();
+    __syncwarp();
+    int old = 0;
+    if (threadIdx.x % 32 == 0) old = atomicAdd(cnt + tile * OZ_EPI_WARPS + w, 1);
+    const bool last = __shfl_sync(0xffffffffu, old, 0) == splits - 1;
+    if (last) __threadfence();
+    return last;
 }
 
 // One CTA computes 128 x BN tiles of the embedded output, in turn for the
@@ -1004,7 +1074,7 @@ __device__ __forceinline__ void oz_gemm_body(const Src &src) {
         return (NI == 2 && (NST & 1)) ? (r >> 1) & 1u : r & 1u;
     };
     const int tid = threadIdx.x, warp = tid / 32, lane = tid % 32;
-    const int64_t T = src.tiles();
+    const int64_t T = src.units();
     int32_t *status;
     {
         int64_t unused;
@@ -1015,6 +1085,8 @@ __device__ __forceinline__ void oz_gemm_body(const Src &src) {
         if (!Src::kTable && a0.sel && *a0.sel != S) return;
         status = a0.status;
     }
+    // likewise a table none of whose contractions chose this count
+    if (!src.any(S)) return;
 
     if (tid == 0) {
         for (int s = 0; s < NST; ++s) {
@@ -1066,10 +1138,8 @@ __device__ __forceinline__ void oz_gemm_body(const Src &src) {
                     t = skip_job(src, hint, t);
                     continue;
                 }
-                int64_t m0, n0;
-                int l;
-                oz_tile(J, local, BN, m0, n0, l);
-                for (int kb = 0; kb < J.a.nkb; ++kb, ++g) {
+                const OzUnit u = oz_unit(J, local, BN);
+                for (int kb = u.kb0; kb < u.kb1; ++kb, ++g) {
                     const int s = (int)(g % NST);
                     const uint32_t round = g / NST;
                     if (!mbar_wait(smem_u32(empty + s), (round & 1) ^ 1, abort_flag, status)) {
@@ -1079,8 +1149,8 @@ __device__ __forceinline__ void oz_gemm_body(const Src &src) {
                     uint8_t *st = smem + s * STAGE;
                     const uint32_t fb = smem_u32(full + full_idx(g));
                     mbar_expect_tx(fb, STAGE);
-                    tma_load_3d(smem_u32(st), &J.tmA, kb * OZ_BK, (int)m0, l * S, fb);
-                    tma_load_3d(smem_u32(st + S * OZ_A_TILE), &J.tmB, kb * OZ_BK, (int)n0, l * S, fb);
+                    tma_load_3d(smem_u32(st), &J.tmA, kb * OZ_BK, (int)u.m0, u.l * S, fb);
+                    tma_load_3d(smem_u32(st + S * OZ_A_TILE), &J.tmB, kb * OZ_BK, (int)u.n0, u.l * S, fb);
                 }
             }
             // make sure no bulk copy is still writing into shared memory
@@ -1106,7 +1176,8 @@ __device__ __forceinline__ void oz_gemm_body(const Src &src) {
                     t = skip_job(src, hint, t);
                     continue;
                 }
-                const int nkb = J.a.nkb, kcb = J.a.kcb;
+                const OzUnit u = oz_unit(J, local, BN);
+                const int nkb = u.kb1 - u.kb0, kcb = J.a.kcb;
                 for (int c0 = 0; c0 < nkb && ok; c0 += kcb, ++C) {
                     const uint32_t bank = C & 1u;
                     if (!mbar_wait(smem_u32(acc_empty + bank), ((C >> 1) & 1u) ^ 1u, abort_flag, status)) {
@@ -1159,11 +1230,11 @@ __device__ __forceinline__ void oz_gemm_body(const Src &src) {
                 continue;
             }
             const OzGemmArgs &args = J.a;
-            int64_t m0, n0;
-            int l;
-            oz_tile(J, local, BN, m0, n0, l);
-            const int64_t row = m0 + 32 * q + lane;
-            const int nchunks = (args.nkb + args.kcb - 1) / args.kcb;
+            const OzUnit u = oz_unit(J, local, BN);
+            const int64_t n0 = u.n0;
+            const int l = u.l;
+            const int64_t row = u.m0 + 32 * q + lane;
+            const int nchunks = (u.kb1 - u.kb0 + args.kcb - 1) / args.kcb;
             // Output addressing of the tile, fetched before the first chunk
             // wait so that its loads overlap the MMAs: the thread's row (offset
             // and exponent), and one output column per lane (lane j < NCOL
@@ -1277,6 +1348,58 @@ __device__ __forceinline__ void oz_gemm_body(const Src &src) {
                 }
             }
             if (!ok) break;
+            if (u.part >= 0) {  // part of a split tile
+                constexpr int NW = EXACT ? 3 * HALF : 2 * HALF;
+                const int w = warp - 2, sp = u.part % args.splits, first = u.part - sp;
+                uint4 *mine = oz_part_at<NW>(args.part, u.part, w);
+#pragma unroll
+                for (int i = 0; i < NW / 4; ++i) {
+                    uint32_t v[4];
+#pragma unroll
+                    for (int e = 0; e < 4; ++e) {
+                        const int k = 4 * i + e;  // a constant: the loops are unrolled
+                        if constexpr (EXACT) v[e] = k < HALF ? w0[k % HALF] : k < 2 * HALF ? w1[k % HALF] : w2[k % HALF];
+                        else v[e] = __float_as_uint(k < HALF ? accf[k % HALF] : comp[k % HALF]);
+                    }
+                    __stcg(mine + i * 32, make_uint4(v[0], v[1], v[2], v[3]));
+                }
+                if (!oz_part_last(args.cnt, u.part / args.splits, w, args.splits)) continue;
+                if constexpr (EXACT) {  // integers: any order gives the same sum
+#pragma unroll 1
+                    for (int o = 0; o < args.splits; ++o) {
+                        if (o == sp) continue;
+                        const uint4 *p = oz_part_at<NW>(args.part, first + o, w);
+#pragma unroll
+                        for (int j0 = 0; j0 < HALF; j0 += 4) {
+                            const uint4 x = __ldcg(p + (j0 / 4) * 32), y = __ldcg(p + ((HALF + j0) / 4) * 32),
+                                        z = __ldcg(p + ((2 * HALF + j0) / 4) * 32);
+                            add96(w0[j0], w1[j0], w2[j0], x.x, y.x, z.x);
+                            add96(w0[j0 + 1], w1[j0 + 1], w2[j0 + 1], x.y, y.y, z.y);
+                            add96(w0[j0 + 2], w1[j0 + 2], w2[j0 + 2], x.z, y.z, z.z);
+                            add96(w0[j0 + 3], w1[j0 + 3], w2[j0 + 3], x.w, y.w, z.w);
+                        }
+                    }
+                } else {  // compensated float sums, always in the order of k
+#pragma unroll
+                    for (int j = 0; j < HALF; ++j) accf[j] = comp[j] = 0.f;
+#pragma unroll 1
+                    for (int o = 0; o < args.splits; ++o) {
+                        const uint4 *p = oz_part_at<NW>(args.part, first + o, w);
+#pragma unroll
+                        for (int j0 = 0; j0 < HALF; j0 += 4) {
+                            const uint4 x = __ldcg(p + (j0 / 4) * 32), y = __ldcg(p + ((HALF + j0) / 4) * 32);
+                            const uint32_t xs[4] = {x.x, x.y, x.z, x.w}, ys[4] = {y.x, y.y, y.z, y.w};
+#pragma unroll
+                            for (int e = 0; e < 4; ++e) {
+                                const float t = __uint_as_float(xs[e]) - (__uint_as_float(ys[e]) + comp[j0 + e]);
+                                const float s2 = accf[j0 + e] + t;
+                                comp[j0 + e] = (s2 - accf[j0 + e]) - t;
+                                accf[j0 + e] = s2;
+                            }
+                        }
+                    }
+                }
+            }
             if constexpr (EXACT) {
                 // Four conversions at a time through the straight-line routine,
                 // so that their integer sequences interleave (one conversion
@@ -1436,6 +1559,53 @@ void ozaki_orient(ContractionPlan &p) {
     p.swapped = true;
 }
 
+// ---- splitting K ---------------------------------------------------------------
+// The tiles of one contraction rarely fill a whole number of waves of the
+// persistent grid, and a long contraction of few rows and columns has fewer
+// tiles than SMs. The tiles of the last, unfilled wave are therefore cut along
+// K into `splits` units each, at most OZ_SPLIT_WAVES waves of them, by the
+// number of units for which that wave is shortest under these times (us),
+// measured on 1 .. 256 tiles of 4 .. 512 k blocks: a k block 0.6 (0.52 with
+// idle SMs, 0.68 without, at S = 6; 1.1 at S = 8) or 0.4 (BF16x3), publishing
+// the sums 2, reading those of one unit 0.4, a second wave of units 8 (its
+// readout waits for the first's sums to leave). One when none is shorter by
+// OZ_SPLIT_GAIN. E.g. one tile of 512 k blocks at S = 6: 279 us whole, 33 in
+// 32 units; 100 tiles of 128: 88 whole, 78 in 3 units; 75 tiles of 8: 16.4
+// whole, 17.9 in 2 units. The rule sees shapes only, so that a contraction is
+// cut the same way alone, in a group and in a served batch, and with every
+// slice count (all exact tiles are equally wide).
+constexpr int OZ_SPLIT_WAVES = 2;
+constexpr double OZ_SPLIT_FIXED = 2.0, OZ_SPLIT_EACH = 0.4, OZ_SPLIT_WAVE = 8.0, OZ_SPLIT_GAIN = 1.0;
+constexpr double oz_kb_us(bool exact) { return exact ? 0.6 : 0.4; }
+static uint64_t oz_part_bytes(bool exact) {
+    return (uint64_t)OZ_BM * oz_bn(exact ? 8 : 3, exact) * (exact ? 12 : 8);
+}
+static int sm_count();
+// Sets the plan's split; returns the number of its units (0: no tile is split).
+static int64_t oz_split(ContractionPlan &p) {
+    const int64_t bn = oz_bn(p.slices, p.form == MGB_FORM_OZAKI);
+    const int64_t tiles = ((p.m_e + OZ_BM - 1) / OZ_BM) * ((p.n_e + bn - 1) / bn) * p.L;
+    const int64_t nkb = (p.k_e + OZ_BK - 1) / OZ_BK, sms = sm_count(), tail = tiles % sms;
+    p.split_full = tiles;
+    p.splits = 1;
+    p.split_kbs = 0;
+    if (tail == 0 || nkb > INT32_MAX / 2) return 0;
+    const double kb = oz_kb_us(p.form == MGB_FORM_OZAKI);
+    double best = nkb * kb - OZ_SPLIT_GAIN;
+    for (int64_t s = 2; s <= OZ_SPLIT_WAVES * sms / tail && s <= nkb; ++s) {
+        const int64_t kbs = (nkb + s - 1) / s, waves = (tail * s + sms - 1) / sms;
+        if ((s - 1) * kbs >= nkb) continue;  // an empty last unit
+        const double t = waves * kbs * kb + (waves - 1) * OZ_SPLIT_WAVE + OZ_SPLIT_FIXED + OZ_SPLIT_EACH * s;
+        if (t < best) {
+            best = t;
+            p.split_full = tiles - tail;
+            p.splits = (int32_t)s;
+            p.split_kbs = (int32_t)kbs;
+        }
+    }
+    return p.splits > 1 ? tail * p.splits : 0;
+}
+
 void ozaki_setup(ContractionPlan &p) {
     bool cx = is_complex(p.compute_dtype);
     if (p.adaptive) {
@@ -1477,7 +1647,20 @@ void ozaki_setup(ContractionPlan &p) {
             off = align256(off + (uint64_t)p.L * ((p.N + 31) / 32) * p.K * 8);
         }
     }
+    p.ws_min = off;
+    if (const int64_t units = oz_split(p)) {
+        p.ws_cnt = off;
+        off = align256(off + units / p.splits * OZ_EPI_WARPS * 4);
+        p.ws_part = off;
+        off = align256(off + units * oz_part_bytes(p.form == MGB_FORM_OZAKI));
+    }
     p.ws_bytes = off;
+}
+
+// Counters of the split tiles (one per tile and epilogue warp).
+static int split_counters(const ContractionPlan &p) {
+    if (p.splits <= 1) return 0;
+    return (int)((p.ws_part - p.ws_cnt) / 4);  // with the padding between the two areas
 }
 
 // Statistics area of an adaptive plan inside the workspace.
@@ -1626,15 +1809,16 @@ static int unit_row_fast(const ModeGroup &gr, const ModeGroup &gk, int t) {
 
 template <typename T, bool BF3>
 static int run_prepass(const OpGeom &g, int mode, const void *X, int32_t *exps, int S, uint32_t *out,
-                       int64_t rows_e, int64_t kw, int64_t L, cudaStream_t s, const int32_t *sel = nullptr) {
+                       int64_t rows_e, int64_t kw, int64_t L, cudaStream_t s, const int32_t *sel = nullptr,
+                       int32_t *cnt = nullptr, int ncnt = 0) {
     int64_t tiles = ((g.R + 31) / 32) * ((g.K + OZ_SLICE_KT - 1) / OZ_SLICE_KT);
     if (tiles > INT32_MAX) return fail(MGB_ERR_UNSUPPORTED, "operand too large for the slicer grid");
     dim3 grid((unsigned)tiles, (unsigned)L);
     const T *x = (const T *)X;
     switch (mode) {
-    case MODE_REAL: k_oz_slice<T, MODE_REAL, BF3><<<grid, 256, 0, s>>>(x, g, exps, S, out, rows_e, kw, sel); break;
-    case MODE_CA: k_oz_slice<T, MODE_CA, BF3><<<grid, 256, 0, s>>>(x, g, exps, S, out, rows_e, kw, sel); break;
-    default: k_oz_slice<T, MODE_CB, BF3><<<grid, 256, 0, s>>>(x, g, exps, S, out, rows_e, kw, sel); break;
+    case MODE_REAL: k_oz_slice<T, MODE_REAL, BF3><<<grid, 256, 0, s>>>(x, g, exps, S, out, rows_e, kw, sel, cnt, ncnt); break;
+    case MODE_CA: k_oz_slice<T, MODE_CA, BF3><<<grid, 256, 0, s>>>(x, g, exps, S, out, rows_e, kw, sel, cnt, ncnt); break;
+    default: k_oz_slice<T, MODE_CB, BF3><<<grid, 256, 0, s>>>(x, g, exps, S, out, rows_e, kw, sel, cnt, ncnt); break;
     }
     MGB_CUDA_CHECK(cudaGetLastError());
     return MGB_OK;
@@ -1674,7 +1858,7 @@ using TypeOf = typename std::remove_pointer<P>::type;
 
 // Pre-pass of the emulated forms: exponents (OZAKI) and slices of A and B
 // into the workspace.
-int ozaki_prepass(const ContractionPlan &p, const void *A, const void *B, void *ws, cudaStream_t s) {
+int ozaki_prepass(const ContractionPlan &p, const void *A, const void *B, void *ws, bool split, cudaStream_t s) {
     if (((uintptr_t)ws & 255) != 0) return fail(MGB_ERR_WORKSPACE, "workspace must be 256-byte aligned");
     const bool exact = p.form == MGB_FORM_OZAKI;
     const bool cx = is_complex(p.compute_dtype);
@@ -1693,6 +1877,9 @@ int ozaki_prepass(const ContractionPlan &p, const void *A, const void *B, void *
     gb.rows_fast = unit_row_fast(p.gn, p.gk, 1);
     const int64_t kw = p.kpad / 2;
     const int mode_a = cx ? MODE_CA : MODE_REAL, mode_b = cx ? MODE_CB : MODE_REAL;
+    int32_t *cnt = nullptr;  // counters of split tiles, cleared with the slicing of A
+    const int ncnt = split ? split_counters(p) : 0;
+    if (ncnt) cnt = (int32_t *)(w + p.ws_cnt);
     int st;
     if (exact) {
         MGB_CUDA_CHECK(cudaMemsetAsync(ea, 0, (size_t)p.L * p.M * 4, s));
@@ -1725,7 +1912,7 @@ int ozaki_prepass(const ContractionPlan &p, const void *A, const void *B, void *
             MGB_CUDA_CHECK(cudaGetLastError());
         }
         st = by_type(p.a.dtype, [&](auto tag) {
-            return run_prepass<TypeOf<decltype(tag)>, false>(ga, mode_a, A, ea, S, sa, p.m_e, kw, p.L, s, sel);
+            return run_prepass<TypeOf<decltype(tag)>, false>(ga, mode_a, A, ea, S, sa, p.m_e, kw, p.L, s, sel, cnt, ncnt);
         });
         if (st) return st;
         st = by_type(p.b.dtype, [&](auto tag) {
@@ -1733,8 +1920,10 @@ int ozaki_prepass(const ContractionPlan &p, const void *A, const void *B, void *
         });
         if (st) return st;
     } else {
-        st = p.a.dtype == MGB_C32 ? run_prepass<float2, true>(ga, mode_a, A, nullptr, 3, sa, p.m_e, kw, p.L, s)
-                                  : run_prepass<float, true>(ga, mode_a, A, nullptr, 3, sa, p.m_e, kw, p.L, s);
+        st = p.a.dtype == MGB_C32 ? run_prepass<float2, true>(ga, mode_a, A, nullptr, 3, sa, p.m_e, kw, p.L, s, nullptr,
+                                                              cnt, ncnt)
+                                  : run_prepass<float, true>(ga, mode_a, A, nullptr, 3, sa, p.m_e, kw, p.L, s, nullptr,
+                                                             cnt, ncnt);
         if (st) return st;
         st = p.b.dtype == MGB_C32 ? run_prepass<float2, true>(gb, mode_b, B, nullptr, 3, sb, p.n_e, kw, p.L, s)
                                   : run_prepass<float, true>(gb, mode_b, B, nullptr, 3, sb, p.n_e, kw, p.L, s);
@@ -1744,7 +1933,8 @@ int ozaki_prepass(const ContractionPlan &p, const void *A, const void *B, void *
 }
 
 // The GEMM's view of a plan whose slices lie in `ws`.
-static int ozaki_job(const ContractionPlan &p, void *C, void *ws, OzJob &job, int64_t &tiles, int S = 0,
+// `split`: the workspace has room for the sums of split tiles (ws_bytes, not only ws_min).
+static int ozaki_job(const ContractionPlan &p, void *C, void *ws, bool split, OzJob &job, int64_t &units, int S = 0,
                      const int32_t *sel = nullptr) {
     const bool exact = p.form == MGB_FORM_OZAKI;
     if (S == 0) S = p.slices;
@@ -1781,21 +1971,33 @@ static int ozaki_job(const ContractionPlan &p, void *C, void *ws, OzJob &job, in
     a.sel = sel;
     if (a.gm.n == 0) { a.gm.n = 1; a.gm.ext[0] = 1; for (int t = 0; t < 3; ++t) a.gm.str[t][0] = 0; }
     if (a.gn.n == 0) { a.gn.n = 1; a.gn.ext[0] = 1; for (int t = 0; t < 3; ++t) a.gn.str[t][0] = 0; }
+    a.full = INT64_MAX;
+    a.splits = 1;
+    a.kbs = a.nkb;
+    if (split && p.splits > 1) {
+        a.full = p.split_full;
+        a.splits = p.splits;
+        a.kbs = p.split_kbs;
+        a.cnt = (int32_t *)(w + p.ws_cnt);
+        a.part = (uint32_t *)(w + p.ws_part);
+    }
     job.tiles_n = (int32_t)((p.n_e + bn - 1) / bn);
     job.tiles_m = (int32_t)((p.M + OZ_BM - 1) / OZ_BM);
     job.L = (int32_t)p.L;
     if ((p.n_e + bn - 1) / bn > INT32_MAX || (p.M + OZ_BM - 1) / OZ_BM > INT32_MAX || p.L > INT32_MAX)
         return fail(MGB_ERR_UNSUPPORTED, "contraction too large for the tile grid");
-    tiles = (int64_t)job.tiles_n * job.tiles_m * job.L;
+    const int64_t all = (int64_t)job.tiles_n * job.tiles_m * job.L;
+    if (a.full > all) a.full = all;
+    units = job.units();
     return MGB_OK;
 }
 
-int ozaki_gemm(const ContractionPlan &p, const void *A, const void *B, void *C, void *ws, cudaStream_t s) {
+int ozaki_gemm(const ContractionPlan &p, const void *A, const void *B, void *C, void *ws, bool split, cudaStream_t s) {
     int st;
     OzJob job;
     int64_t tiles = 0;
     if (!p.adaptive) {
-        if ((st = ozaki_job(p, C, ws, job, tiles))) return st;
+        if ((st = ozaki_job(p, C, ws, split, job, tiles))) return st;
         return launch_gemm(p.slices, p.form == MGB_FORM_OZAKI, is_complex(p.compute_dtype), job, tiles, s);
     }
     // Every candidate is launched; the kernel of the chosen count works and
@@ -1803,18 +2005,18 @@ int ozaki_gemm(const ContractionPlan &p, const void *A, const void *B, void *C, 
     const int32_t *sel = &stat_area(p, ws).st->sel;
     for (int S = 3; S <= 8; ++S) {
         if (!(p.cand_mask & (1u << S))) continue;
-        if ((st = ozaki_job(p, C, ws, job, tiles, S, sel))) return st;
+        if ((st = ozaki_job(p, C, ws, split, job, tiles, S, sel))) return st;
         if ((st = launch_gemm(S, true, is_complex(p.compute_dtype), job, tiles, s))) return st;
     }
     return launch_plain_gemm(p, A, B, C, s, sel);
 }
 
 int launch_ozaki(const ContractionPlan &p, const void *A, const void *B, void *C, void *ws,
-                 cudaStream_t s, cudaEvent_t mid) {
-    int st = ozaki_prepass(p, A, B, ws, s);
+                 bool split, cudaStream_t s, cudaEvent_t mid) {
+    int st = ozaki_prepass(p, A, B, ws, split, s);
     if (st) return st;
     if (mid) MGB_CUDA_CHECK(cudaEventRecord(mid, s));
-    return ozaki_gemm(p, A, B, C, ws, s);
+    return ozaki_gemm(p, A, B, C, ws, split, s);
 }
 
 int ozaki_adaptive_report(const ContractionPlan &p, const void *ws, cudaStream_t s, mgb_adaptive_report *out) {
@@ -1869,8 +2071,8 @@ int ozaki_grouped_create(const std::vector<const ContractionPlan *> &plans, cons
         }
         int64_t t = 0;
         // an adaptive plan's job works only when its device choice is S
-        const int st = p.adaptive ? ozaki_job(p, nullptr, ws[i], host[i], t, S, &stat_area(p, ws[i]).st->sel)
-                                  : ozaki_job(p, nullptr, ws[i], host[i], t);
+        const int st = p.adaptive ? ozaki_job(p, nullptr, ws[i], true, host[i], t, S, &stat_area(p, ws[i]).st->sel)
+                                  : ozaki_job(p, nullptr, ws[i], true, host[i], t);
         if (st) {
             delete g;
             return st;
@@ -1931,6 +2133,8 @@ struct PreJob {
     OzStats *st;        // its statistics (adaptive) or null
     float *q, *P;       // this operand's per-k norms and squared scales
     int2 *part;         // the exponent scan's partials of this operand (adaptive) or null
+    int32_t *cnt;       // counters of split tiles, cleared by the slicing (A's job) or null
+    int32_t ncnt;
     void *zero[2];      // regions cleared by PRE_ZERO (exponents; statistics for t == 0)
     int64_t zero_words[2];
     int64_t tiles[PRE_PHASES];  // blocks of every phase
@@ -2069,6 +2273,7 @@ __global__ void __launch_bounds__(256, 4) k_oz_slice_multi(const PreJob *__restr
         if (S == 0) return;  // the plain form will run this contraction
     }
     const int64_t local = blockIdx.x - start[j];
+    if (local == 0) oz_clear_counters(J.cnt, J.ncnt);
     const int64_t per_l = J.tiles[PRE_SLICE] / max(J.L, 1);
     const int64_t l = local / per_l;
     oz_slice_tile<T, MODE, BF3>((const T *)J.X, J.g, J.exps, S, J.out, J.rows_e, J.kw, local - l * per_l, l, sm);
@@ -2134,7 +2339,7 @@ static int batch_reserve(OzBatchBuffers *b, size_t bytes) {
     return MGB_OK;
 }
 
-static void fill_prejob(PreJob &J, const ContractionPlan &p, int t, const void *X, void *ws) {
+static void fill_prejob(PreJob &J, const ContractionPlan &p, int t, const void *X, void *ws, bool split) {
     std::memset(&J, 0, sizeof(J));
     const bool cx = is_complex(p.compute_dtype), exact = p.form == MGB_FORM_OZAKI;
     uint8_t *w = (uint8_t *)ws;
@@ -2158,6 +2363,10 @@ static void fill_prejob(PreJob &J, const ContractionPlan &p, int t, const void *
     J.out = (uint32_t *)(w + (t == 0 ? p.ws_a : p.ws_b));
     J.rows_e = t == 0 ? p.m_e : p.n_e;
     J.kw = p.kpad / 2;
+    if (t == 0 && split && split_counters(p)) {
+        J.cnt = (int32_t *)(w + p.ws_cnt);
+        J.ncnt = split_counters(p);
+    }
     const int64_t R = J.g.R, K = p.K, L = p.L;
     int64_t zw = 0;
     if (exact) {
@@ -2214,8 +2423,8 @@ static int pre_tables(const std::vector<OzBatchItem> &items, std::vector<PreJob>
         const ContractionPlan &p = *it.p;
         if (p.form == MGB_FORM_PLAIN) return fail(MGB_ERR_ARGUMENT, "batch: plain-form plans are not batched");
         if (((uintptr_t)it.ws & 255) != 0) return fail(MGB_ERR_WORKSPACE, "batch: workspace must be 256-byte aligned");
-        fill_prejob(pre[2 * i], p, 0, p.swapped ? it.B : it.A, it.ws);
-        fill_prejob(pre[2 * i + 1], p, 1, p.swapped ? it.A : it.B, it.ws);
+        fill_prejob(pre[2 * i], p, 0, p.swapped ? it.B : it.A, it.ws, it.split);
+        fill_prejob(pre[2 * i + 1], p, 1, p.swapped ? it.A : it.B, it.ws, it.split);
         if (p.adaptive) choose.push_back(choose_job(p, it.ws));
     }
     // operand jobs of one (form, element type, embedding) lie together: the
@@ -2398,13 +2607,13 @@ int ozaki_batch_launch(const std::vector<OzBatchItem> &items, OzBatchBuffers *bu
                 if (!(p.cand_mask & (1u << S))) continue;
                 OzJob job;
                 int64_t tiles;
-                if (int st = ozaki_job(p, it.C, it.ws, job, tiles, S, &a.st->sel)) return st;
+                if (int st = ozaki_job(p, it.C, it.ws, it.split, job, tiles, S, &a.st->sel)) return st;
                 gem[std::make_tuple(S, 1, cx ? 1 : 0)].push_back(job);
             }
         } else {
             OzJob job;
             int64_t tiles;
-            if (int st = ozaki_job(p, it.C, it.ws, job, tiles)) return st;
+            if (int st = ozaki_job(p, it.C, it.ws, it.split, job, tiles)) return st;
             gem[std::make_tuple(exact ? p.slices : 3, exact ? 1 : 0, cx ? 1 : 0)].push_back(job);
         }
     }
@@ -2447,7 +2656,7 @@ int ozaki_batch_launch(const std::vector<OzBatchItem> &items, OzBatchBuffers *bu
         int64_t *st = (int64_t *)(h + o_gs[vi]);
         st[0] = 0;
         for (size_t j = 0; j < kv.second.size(); ++j)
-            st[j + 1] = st[j] + (int64_t)kv.second[j].tiles_n * kv.second[j].tiles_m * kv.second[j].L;
+            st[j + 1] = st[j] + kv.second[j].units();
         vtiles.push_back(st[kv.second.size()]);
         ++vi;
     }

@@ -49,6 +49,7 @@ struct Req {
     mgb_plan plan;
     const void *A, *B;
     void *C;
+    uint64_t ws;         // workspace bytes
     uint64_t bytes;      // admitted bytes: caller-declared resident bytes + workspace
     cudaEvent_t dep;     // caller-stream event the request waits on (or null)
     Clock::time_point t0;
@@ -150,7 +151,7 @@ static int launch_emulated(mgb_server_s *s, size_t k) {
     uint64_t total = 0;
     for (size_t i = 0; i < b.emu.size(); ++i) {
         off[i] = total;
-        total += (b.emu[i].plan->cp.ws_bytes + 255) & ~uint64_t(255);
+        total += (b.emu[i].ws + 255) & ~uint64_t(255);
     }
     if (b.sel_cap < b.emu.size()) {
         if (b.sel_dev) cudaFree(b.sel_dev);
@@ -166,7 +167,8 @@ static int launch_emulated(mgb_server_s *s, size_t k) {
     if (rc) return rc;
     std::vector<OzBatchItem> items(b.emu.size());
     for (size_t i = 0; i < b.emu.size(); ++i)
-        items[i] = {&b.emu[i].plan->cp, b.emu[i].A, b.emu[i].B, b.emu[i].C, (char *)b.ws + off[i]};
+        items[i] = {&b.emu[i].plan->cp, b.emu[i].A, b.emu[i].B, b.emu[i].C, (char *)b.ws + off[i],
+                    b.emu[i].ws >= b.emu[i].plan->cp.ws_bytes};
     int nv = 0;
     rc = ozaki_batch_launch(
         items, b.buf, st, b.sel_dev,
@@ -259,8 +261,8 @@ static bool retire(mgb_server_s *s, size_t k) {
                 continue;
             }
             void *ws = nullptr;
-            int rc = alloc_ws(s, &ws, r.plan->cp.ws_bytes, st);
-            if (rc == MGB_OK) rc = mgb_contract(r.plan, r.A, r.B, r.C, ws, r.plan->cp.ws_bytes, st);
+            int rc = alloc_ws(s, &ws, r.ws, st);
+            if (rc == MGB_OK) rc = mgb_contract(r.plan, r.A, r.B, r.C, ws, r.ws, st);
             if (ws) cudaFreeAsync(ws, st);
             r.status = rc;
             r.done = take_event(s);
@@ -411,7 +413,9 @@ int mgb_server_submit(mgb_server server, mgb_plan plan, const void *A, const voi
     r.A = A;
     r.B = B;
     r.C = C;
-    r.bytes = resident_bytes + plan->cp.ws_bytes;
+    // a request that the whole budget holds only without split tiles runs without them
+    r.ws = resident_bytes + plan->cp.ws_bytes <= server->budget ? plan->cp.ws_bytes : plan->cp.ws_min;
+    r.bytes = resident_bytes + r.ws;
     r.dep = nullptr;
     r.t0 = Clock::now();
     std::lock_guard<std::mutex> lk(server->mu);
