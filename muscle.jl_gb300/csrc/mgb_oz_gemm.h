@@ -1,6 +1,8 @@
 // The tensor-core GEMM of the emulated forms over digit slices (OZAKI) or
-// pieces (BF16X3), shared by its translation units: one contraction
-// (mgb_oz_gemm_one.cu) and a table of them (mgb_oz_gemm_table.cu).
+// pieces (BF16X3), shared by its translation units: one contraction of a
+// fixed slice count (mgb_oz_gemm_one.cu), one whose slice count the device
+// chose (mgb_oz_gemm_any.cu), and a table of contractions
+// (mgb_oz_gemm_table.cu).
 #pragma once
 
 #include <cuda.h>
@@ -50,6 +52,8 @@ __host__ __device__ constexpr int oz_stage_bytes(int S, bool exact) { return S *
 // for d <= 15. Both hold about the same number of mantissa bits (W S = 48 / 49).
 __host__ __device__ constexpr int oz_digit_bits(int S) { return S <= 6 ? 8 : 7; }
 __host__ __device__ constexpr int oz_chunk_blocks(int S) { return oz_digit_bits(S) == 8 ? 4 : 8; }
+// k blocks between readouts
+__host__ __device__ constexpr int oz_chunk(int S, bool exact) { return exact ? oz_chunk_blocks(S) : OZ_KC / OZ_BK; }
 __host__ __device__ constexpr int oz_stages(int S, bool exact) {
     return (OZ_SMEM_BUDGET / oz_stage_bytes(S, exact)) < OZ_MAX_STAGES ? (OZ_SMEM_BUDGET / oz_stage_bytes(S, exact))
                                                                        : OZ_MAX_STAGES;
@@ -155,13 +159,10 @@ __host__ __device__ constexpr uint32_t oz_idesc(int n) {
 struct OzGemmArgs {
     int64_t M, Ne, N;      // rows of A, embedded rows of B, un-embedded N
     int32_t nkb;           // number of 32-wide k blocks
-    int32_t kcb;           // k blocks per chunk (exact readout interval)
-    int32_t S;             // slices (digits / pieces)
     const int32_t *expA;   // [L][M] biased exponents (OZAKI)
     const int32_t *expB;   // [L][N]
     void *C;
     void *const *cptr;     // per-batch-entry output pointers (grouped execution) or null
-    int32_t band;          // row tiles per rasterisation band
     ModeGroup gm, gn, gl;  // C offsets live in tensor slot 2
     int32_t *status;
     const int32_t *sel;    // adaptive choice (nullable): run only when it holds S
@@ -178,14 +179,24 @@ struct OzGemmArgs {
 // One contraction (or one bucket of a group) as the GEMM sees it: the slice
 // tensor maps, the arguments and its tile grid (column tiles x row tiles x
 // batch entries).
-struct OzJob {  // aligned as its tensor maps
-    CUtensorMap tmA, tmB;
+struct OzJobShape {
     OzGemmArgs a;
     int32_t tiles_n, tiles_m, L;
     __host__ __device__ int64_t units() const {
         const int64_t t = (int64_t)tiles_n * tiles_m * L;
         return a.full + (t - a.full) * a.splits;
     }
+};
+struct OzJob : OzJobShape {  // aligned as its tensor maps
+    CUtensorMap tmA, tmB;
+    int32_t band;  // row tiles per rasterisation band
+};
+// A contraction whose slice count a.sel holds: the tensor maps and the band of
+// every candidate count (3 .. 8), and the candidates (bit S).
+struct OzAnyJob : OzJobShape {
+    CUtensorMap tm[6][2];
+    int32_t band[6];
+    uint32_t cand;
 };
 
 // Tile sources of the kernel: one job in the parameter space, or a table of
@@ -198,10 +209,27 @@ struct OzOneJob {
     const OzJob *j;
     __device__ int64_t units() const { return j->units(); }
     __device__ bool any(int) const { return true; }
-    __device__ const OzJob &job(int64_t t, int64_t &local, int &) const {
+    __device__ const OzJobShape &job(int64_t t, int64_t &local, int &) const {
         local = t;
         return *j;
     }
+    __device__ const CUtensorMap *map_a(int) const { return &j->tmA; }
+    __device__ const CUtensorMap *map_b(int) const { return &j->tmB; }
+    __device__ int band(int) const { return j->band; }
+};
+template <int S>
+struct OzChosenJob {
+    static constexpr bool kTable = false;
+    const OzAnyJob *j;
+    __device__ int64_t units() const { return j->units(); }
+    __device__ bool any(int) const { return true; }
+    __device__ const OzJobShape &job(int64_t t, int64_t &local, int &) const {
+        local = t;
+        return *j;
+    }
+    __device__ const CUtensorMap *map_a(int) const { return &j->tm[S - 3][0]; }
+    __device__ const CUtensorMap *map_b(int) const { return &j->tm[S - 3][1]; }
+    __device__ int band(int) const { return j->band[S - 3]; }
 };
 struct OzJobTable {
     static constexpr bool kTable = true;  // jobs may carry their own adaptive choice (skipped unless it is S)
@@ -214,7 +242,10 @@ struct OzJobTable {
         for (int i = threadIdx.x; i < n; i += blockDim.x) mine = mine || !jobs[i].a.sel || *jobs[i].a.sel == S;
         return __syncthreads_or(mine);
     }
-    __device__ const OzJob &job(int64_t t, int64_t &local, int &hint) const {
+    __device__ const CUtensorMap *map_a(int i) const { return &jobs[i].tmA; }
+    __device__ const CUtensorMap *map_b(int i) const { return &jobs[i].tmB; }
+    __device__ int band(int i) const { return jobs[i].band; }
+    __device__ const OzJobShape &job(int64_t t, int64_t &local, int &hint) const {
         int lo = hint;  // the last job with start <= t, at or after the hint
         if (lo + 1 < n && start[lo + 1] <= t) {
             ++lo;
@@ -266,8 +297,9 @@ __device__ __forceinline__ void oz_tile_t(I local, I nn, I nm, I gm, int bn, int
     m0 = (int64_t)(first + r % rows) * OZ_BM;
     n0 = (int64_t)(r / rows) * bn;
 }
-__device__ __forceinline__ void oz_tile(const OzJob &J, int64_t local, int bn, int64_t &m0, int64_t &n0, int &l) {
-    const int64_t nn = J.tiles_n, nm = J.tiles_m, gm = J.a.band;
+__device__ __forceinline__ void oz_tile(const OzJobShape &J, int64_t local, int64_t gm, int bn, int64_t &m0, int64_t &n0,
+                                        int &l) {
+    const int64_t nn = J.tiles_n, nm = J.tiles_m;
     // 32-bit divisions whenever the job's tile numbers fit (a 64-bit division
     // is a long software sequence)
     if (local <= INT32_MAX && (int64_t)J.L * nn * nm <= INT32_MAX && gm * nn <= INT32_MAX)
@@ -283,7 +315,7 @@ struct OzUnit {
     int64_t m0, n0;
     int l, kb0, kb1, part;
 };
-__device__ __forceinline__ OzUnit oz_unit(const OzJob &J, int64_t local, int bn) {
+__device__ __forceinline__ OzUnit oz_unit(const OzJobShape &J, int64_t local, int band, int bn) {
     OzUnit u;
     u.kb0 = 0;
     u.kb1 = J.a.nkb;
@@ -295,7 +327,7 @@ __device__ __forceinline__ OzUnit oz_unit(const OzJob &J, int64_t local, int bn)
         u.kb1 = min(J.a.nkb, u.kb0 + J.a.kbs);
         local = J.a.full + t;
     }
-    oz_tile(J, local, bn, u.m0, u.n0, u.l);
+    oz_tile(J, local, band, bn, u.m0, u.n0, u.l);
     return u;
 }
 
@@ -336,6 +368,7 @@ __device__ __forceinline__ bool oz_part_last(int32_t *cnt, int tile, int w, int 
 template <int S, bool EXACT, bool CX, typename Src>
 __device__ __forceinline__ void oz_gemm_body(const Src &src) {
     constexpr int W = oz_digit_bits(S);  // digit width (EXACT)
+    constexpr int KCB = oz_chunk(S, EXACT);  // k blocks per chunk
     constexpr int NST = oz_stages(S, EXACT);
     constexpr int STAGE = oz_stage_bytes(S, EXACT);
     constexpr int BN = oz_bn(S, EXACT);  // columns per digit group, embedded B rows per CTA
@@ -387,12 +420,10 @@ __device__ __forceinline__ void oz_gemm_body(const Src &src) {
         int64_t unused;
         int h0 = 0;
         const OzGemmArgs &a0 = src.job(0, unused, h0).a;
-        // an adaptive plan launches every candidate; all but the chosen one
-        // return before touching shared memory or TMEM
-        if (!Src::kTable && a0.sel && *a0.sel != S) return;
         status = a0.status;
     }
-    // likewise a table none of whose contractions chose this count
+    // a table none of whose contractions chose this count returns before it
+    // touches shared memory or TMEM
     if (!src.any(S)) return;
 
     if (tid == 0) {
@@ -440,12 +471,12 @@ __device__ __forceinline__ void oz_gemm_body(const Src &src) {
             int hint = 0;
             for (int64_t t = blockIdx.x; t < T && ok; t += gridDim.x) {
                 int64_t local;
-                const OzJob &J = src.job(t, local, hint);
+                const OzJobShape &J = src.job(t, local, hint);
                 if (Src::kTable && J.a.sel && *J.a.sel != S) {  // a job of another slice count
                     t = skip_job(src, hint, t);
                     continue;
                 }
-                const OzUnit u = oz_unit(J, local, BN);
+                const OzUnit u = oz_unit(J, local, src.band(hint), BN);
                 for (int kb = u.kb0; kb < u.kb1; ++kb, ++g) {
                     const int s = (int)(g % NST);
                     const uint32_t round = g / NST;
@@ -456,8 +487,8 @@ __device__ __forceinline__ void oz_gemm_body(const Src &src) {
                     uint8_t *st = smem + s * STAGE;
                     const uint32_t fb = smem_u32(full + full_idx(g));
                     mbar_expect_tx(fb, STAGE);
-                    tma_load_3d(smem_u32(st), &J.tmA, kb * OZ_BK, (int)u.m0, u.l * S, fb);
-                    tma_load_3d(smem_u32(st + S * OZ_A_TILE), &J.tmB, kb * OZ_BK, (int)u.n0, u.l * S, fb);
+                    tma_load_3d(smem_u32(st), src.map_a(hint), kb * OZ_BK, (int)u.m0, u.l * S, fb);
+                    tma_load_3d(smem_u32(st + S * OZ_A_TILE), src.map_b(hint), kb * OZ_BK, (int)u.n0, u.l * S, fb);
                 }
             }
             // make sure no bulk copy is still writing into shared memory
@@ -478,20 +509,20 @@ __device__ __forceinline__ void oz_gemm_body(const Src &src) {
             int hint = 0;
             for (int64_t t = blockIdx.x; t < T && ok; t += gridDim.x) {
                 int64_t local;
-                const OzJob &J = src.job(t, local, hint);
+                const OzJobShape &J = src.job(t, local, hint);
                 if (Src::kTable && J.a.sel && *J.a.sel != S) {  // a job of another slice count
                     t = skip_job(src, hint, t);
                     continue;
                 }
-                const OzUnit u = oz_unit(J, local, BN);
-                const int nkb = u.kb1 - u.kb0, kcb = J.a.kcb;
-                for (int c0 = 0; c0 < nkb && ok; c0 += kcb, ++C) {
+                const OzUnit u = oz_unit(J, local, src.band(hint), BN);
+                const int nkb = u.kb1 - u.kb0;
+                for (int c0 = 0; c0 < nkb && ok; c0 += KCB, ++C) {
                     const uint32_t bank = C & 1u;
                     if (!mbar_wait(smem_u32(acc_empty + bank), ((C >> 1) & 1u) ^ 1u, abort_flag, status)) {
                         ok = false;
                         break;
                     }
-                    const int c1 = min(nkb, c0 + kcb);
+                    const int c1 = min(nkb, c0 + KCB);
                     for (int kb = c0; kb < c1; ++kb) {
                         const uint32_t gg = g + (uint32_t)kb;
                         if (NI == 2 && (int)(gg & 1u) != me) continue;
@@ -531,17 +562,17 @@ __device__ __forceinline__ void oz_gemm_body(const Src &src) {
         int hint = 0;
         for (int64_t t = blockIdx.x; t < T && ok; t += gridDim.x) {
             int64_t local;
-            const OzJob &J = src.job(t, local, hint);
+            const OzJobShape &J = src.job(t, local, hint);
             if (Src::kTable && J.a.sel && *J.a.sel != S) {  // a job of another slice count
                 t = skip_job(src, hint, t);
                 continue;
             }
             const OzGemmArgs &args = J.a;
-            const OzUnit u = oz_unit(J, local, BN);
+            const OzUnit u = oz_unit(J, local, src.band(hint), BN);
             const int64_t n0 = u.n0;
             const int l = u.l;
             const int64_t row = u.m0 + 32 * q + lane;
-            const int nchunks = (u.kb1 - u.kb0 + args.kcb - 1) / args.kcb;
+            const int nchunks = (u.kb1 - u.kb0 + KCB - 1) / KCB;
             // Output addressing of the tile, fetched before the first chunk
             // wait so that its loads overlap the MMAs: the thread's row (offset
             // and exponent), and one output column per lane (lane j < NCOL
@@ -830,6 +861,9 @@ inline int set_smem_attr(K kern, int smem, std::atomic<bool> (&done)[OZ_MAX_DEVI
 // The contraction of `job`, on a persistent grid (one CTA per SM, each
 // walking its share of the units).
 int oz_launch_one(int S, bool exact, bool cx, const OzJob &job, int64_t units, cudaStream_t s);
+// The contraction of `job` with the slice count that the device chose (exact
+// form; nothing when that is 0, the plain form).
+int oz_launch_any(bool cx, const OzAnyJob &job, int64_t units, cudaStream_t s);
 // Every contraction of a device table of one kernel variant.
 int oz_launch_table(int S, bool exact, bool cx, const OzJob *jobs, const int64_t *start, int njobs, int64_t units,
                     cudaStream_t s);

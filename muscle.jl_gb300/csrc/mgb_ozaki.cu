@@ -231,11 +231,48 @@ __device__ __forceinline__ void oz_scale_tile(const T *__restrict__ X, const OpG
         }
     }
 }
+
+// Both operands of one contraction (or of one bucket of a group), as the
+// pre-pass launches see them. Blocks [0, tiles) of a launch work on op[0],
+// the rest on op[1]: one launch per phase instead of one per operand, since a
+// small contraction's pre-pass is launches and little else (`only` >= 0: the
+// launch covers that operand alone, when their element types differ).
+struct PreOperand {
+    OpGeom g;
+    const void *X;
+    int32_t *exps;      // [L][R] (Ozaki)
+    int2 *part;         // the exponent scan's partials (adaptive) or null
+    uint32_t *out;      // slice planes
+    int64_t rows_e;
+    int64_t tiles;      // 32-row x 64-k tiles per batch entry
+};
+struct OzStats;
+struct PrePair {
+    PreOperand op[2];
+    int32_t *emax;        // [2] largest exponents (adaptive) or null
+    int64_t kw;
+    const int32_t *sel;   // adaptive choice or null
+    int32_t S;            // slice count when `sel` is null
+    int32_t ncnt;
+    int32_t *cnt;         // counters of split tiles, cleared by the slicing, or null
+};
+static_assert(sizeof(PrePair) + 16 <= 4096, "kernel parameters");
+// The operand of this block, and the block's tile of it.
+__device__ __forceinline__ int pre_operand(const PrePair &a, int only, int64_t &blk) {
+    blk = blockIdx.x;
+    if (only >= 0) return only;
+    if (blk < a.op[0].tiles) return 0;
+    blk -= a.op[0].tiles;
+    return 1;
+}
+
 template <typename T>
-__global__ void __launch_bounds__(256, 4) k_oz_scale(const T *__restrict__ X, OpGeom g, int32_t *exps, int32_t *emax,
-                                                  int2 *part) {
+__global__ void __launch_bounds__(256, 4) k_oz_scale(const __grid_constant__ PrePair a, int only) {
     __shared__ ScaleSmem sm;
-    oz_scale_tile<T>(X, g, exps, emax, part, blockIdx.x, blockIdx.y, sm);
+    int64_t blk;
+    const int o = pre_operand(a, only, blk);
+    const PreOperand &p = a.op[o];
+    oz_scale_tile<T>((const T *)p.X, p.g, p.exps, a.emax ? a.emax + o : nullptr, p.part, blk, blockIdx.y, sm);
 }
 
 // =============================================================================
@@ -262,7 +299,8 @@ struct OzStats {
     int32_t nonfinite;  // an operand holds Inf / NaN
     int32_t emax[2];    // largest biased exponent of A and B
     float est[9];       // estimated error per candidate slice count
-    int32_t pad[3];
+    uint32_t blocks;    // blocks of k_oz_stat that are done
+    int32_t pad[2];
     // sums over k and batch entries (cleared with the header every call):
     // P_A sum q_B + P_B sum q_A, sum q_A q_B, K P_A P_B
     double acc[3];
@@ -316,11 +354,6 @@ __device__ __forceinline__ void oz_stat_block(const int2 *__restrict__ part, con
         if (s2 != 0.f) atomicAdd(P + l, s2);
     }
 }
-__global__ void __launch_bounds__(256) k_oz_stat(const int2 *__restrict__ part, const int32_t *__restrict__ exps,
-                                                 OzStats *st, int t, float *q, float *P, int64_t R, int64_t K) {
-    __shared__ StatSmem sm;
-    oz_stat_block(part, exps, st, t, q, P, R, K, blockIdx.x, blockIdx.y, sm);
-}
 __host__ __device__ inline int64_t oz_stat_blocks(int64_t R, int64_t K) { return (K + 255) / 256 + (R + 255) / 256; }
 
 // The sums behind the estimate, spread over the GPU: block b of batch entry
@@ -364,38 +397,156 @@ __device__ __forceinline__ void oz_est_block(OzStats *st, const float *__restric
         if (blk == 0 && Pa * Pb != 0.0) atomicAdd(&st->acc[2], (double)K * Pa * Pb);
     }
 }
-__global__ void __launch_bounds__(256) k_oz_est(OzStats *st, const float *__restrict__ qa, const float *__restrict__ qb,
-                                                const float *__restrict__ pa, const float *__restrict__ pb, int64_t K) {
-    __shared__ double red[2][8];
-    const int64_t nb = oz_est_blocks(K), l = blockIdx.x / nb;
-    oz_est_block(st, qa, qb, pa, pb, K, blockIdx.x - l * nb, l, red);
-}
-
-// One thread: the error estimate of every candidate slice count (bit S of
-// `cand`) from the sums, and the choice, the smallest count within `tol`,
-// else 0 (plain).
-__device__ __forceinline__ void oz_choose_final(OzStats *st, uint32_t cand, double tol, double margin, int cx) {
-    const double trunc = st->acc[0], den = st->acc[1], drop = st->acc[2];
-    const double f1 = cx ? 2.0 : 1.0, f2 = cx ? 4.0 : 1.0;
-    int sel = 0;
-    for (int S = 8; S >= 1; --S) {
-        st->est[S] = 0.f;
-        if (!(cand & (1u << S))) continue;
+// One warp: the error estimate of every candidate slice count (bit S of
+// `cand`, lane S) from the sums, and the choice, the smallest count within
+// `tol`, else 0 (plain).
+__device__ __forceinline__ void oz_choose_warp(OzStats *st, double trunc, double den, double drop, uint32_t cand,
+                                               double tol, double margin, int cx) {
+    const int S = threadIdx.x % 32;
+    const bool is = S >= 1 && S <= 8 && (cand & (1u << S));
+    double e = 0.0;
+    if (is) {
+        const double f1 = cx ? 2.0 : 1.0, f2 = cx ? 4.0 : 1.0;
         const int W = S <= 6 ? 8 : 7;
-        const double u = ldexp(1.0, -W * S);
+        const double u = __longlong_as_double((long long)(1023 - W * S) << 52);
         const double num = u * u * (f1 / 12.0 * trunc + f2 * (S - 1) / 144.0 * drop);
-        double e;
         if (num == 0.0) e = 0.0;                 // an operand is zero: every form is exact
         else if (den == 0.0) e = INFINITY;       // no overlap the estimate can rest on
         else e = sqrt(num / den) * margin;
-        st->est[S] = (float)e;
-        if (e <= tol && !st->nonfinite) sel = S;  // scanning down: ends at the smallest
     }
-    st->est[0] = 0.f;
-    st->sel = sel;
+    const bool fin = __ldcg(&st->nonfinite) == 0;
+    const uint32_t ok = __ballot_sync(0xffffffffu, is && e <= tol && fin);
+    if (S <= 8) st->est[S] = is ? (float)e : 0.f;
+    if (S == 0) st->sel = ok ? __ffs(ok) - 1 : 0;
 }
-__global__ void k_oz_choose(OzStats *st, uint32_t cand, double tol, double margin, int cx) {
-    if (threadIdx.x == 0) oz_choose_final(st, cand, tol, margin, cx);
+
+// Statistics, estimate and choice of one contraction in one launch. Blocks
+// [0, ceil(K / 32)) of batch entry l sum the scan's partials of both operands
+// over their row tiles (a warp takes every eighth one, so that few k still
+// fill the GPU) and add the entry's sum of q_A, of q_B and of q_A q_B; the
+// blocks after them add the rows' squared scales to P and flag non-finite
+// rows; the block that finishes last chooses.
+constexpr int OZ_STAT_K = 32;
+struct StatArgs {
+    const int2 *part[2];
+    const int32_t *exps[2];
+    int64_t R[2], K, L;
+    OzStats *st;
+    float *P[2];   // [L]
+    // [L] sums of q: doubles, or floats for K = 1, whose one q per entry is the
+    // sum (the area holds one float per entry and k)
+    void *Q[2];
+    double tol, margin;
+    uint32_t cand;
+    int32_t cx;
+};
+__host__ __device__ inline int64_t oz_stat_grid(int64_t R0, int64_t R1, int64_t K) {
+    return (K + OZ_STAT_K - 1) / OZ_STAT_K + (R0 + 255) / 256 + (R1 + 255) / 256;
+}
+__global__ void __launch_bounds__(256) k_oz_stat(const __grid_constant__ StatArgs a) {
+    __shared__ float red[2][8][33];
+    __shared__ double dred[2][8];
+    __shared__ int last;
+    const int64_t nq = (a.K + OZ_STAT_K - 1) / OZ_STAT_K, l = blockIdx.y;
+    const int warp = threadIdx.x / 32, lane = threadIdx.x % 32;
+    int64_t blk = blockIdx.x;
+    if (blk < nq) {
+        const int64_t k = blk * OZ_STAT_K + lane;
+#pragma unroll
+        for (int t = 0; t < 2; ++t) {
+            const int64_t R32 = (a.R[t] + 31) / 32;
+            const int be_max = a.st->emax[t];
+            const int2 *p = a.part[t] + l * R32 * a.K + k;
+            float acc = 0.f;
+            if (k < a.K)
+#pragma unroll 4
+                for (int64_t tr = warp; tr < R32; tr += 8) {
+                    const int2 v = __ldg(p + tr * a.K);
+                    const float x = __int_as_float(v.y);
+                    if (x != 0.f) acc += x * pow4f(v.x - be_max - 1);
+                }
+            red[t][warp][lane] = acc;
+        }
+        __syncthreads();
+        if (warp < 3) {  // the sums of q_A, of q_B, of q_A q_B
+            float q[2] = {0.f, 0.f};
+#pragma unroll
+            for (int y = 0; y < 8; ++y) {
+                q[0] += red[0][y][lane];
+                q[1] += red[1][y][lane];
+            }
+            double v = warp == 0 ? (double)q[0] : warp == 1 ? (double)q[1] : (double)q[0] * q[1];
+#pragma unroll
+            for (int d = 16; d > 0; d >>= 1) v += __shfl_xor_sync(0xffffffffu, v, d);
+            if (lane == 0) {
+                if (warp == 2) {
+                    if (v != 0.0) atomicAdd(&a.st->acc[1], v);
+                } else if (a.K == 1) {
+                    ((float *)a.Q[warp])[l] = (float)v;
+                } else if (v != 0.0) {
+                    atomicAdd((double *)a.Q[warp] + l, v);
+                }
+            }
+        }
+    } else {
+        blk -= nq;
+        const int64_t nr0 = (a.R[0] + 255) / 256;
+        const int t = blk >= nr0;
+        const int64_t i = (t ? blk - nr0 : blk) * 256 + threadIdx.x;
+        float w = 0.f;
+        if (i < a.R[t]) {
+            const int be = a.exps[t][l * a.R[t] + i];
+            if (be == 0x7FF) a.st->nonfinite = 1;
+            else if (be > 0) w = pow4f(be - a.st->emax[t]);
+        }
+#pragma unroll
+        for (int d = 16; d > 0; d >>= 1) w += __shfl_xor_sync(0xffffffffu, w, d);
+        if (lane == 0) red[0][0][warp] = w;
+        __syncthreads();
+        if (threadIdx.x == 0) {
+            float s2 = 0.f;
+            for (int y = 0; y < 8; ++y) s2 += red[0][0][y];
+            if (s2 != 0.f) atomicAdd(a.P[t] + l, s2);
+        }
+    }
+    __threadfence();
+    __syncthreads();
+    if (threadIdx.x == 0) {
+        last = atomicAdd(&a.st->blocks, 1u) + 1u == gridDim.x * gridDim.y;
+        __threadfence();
+    }
+    __syncthreads();
+    if (!last) return;
+    auto sum_q = [&](int t, int64_t i) {
+        return a.K == 1 ? (double)__ldcg((const float *)a.Q[t] + i) : __ldcg((const double *)a.Q[t] + i);
+    };
+    double tr = 0.0, drop = 0.0;
+    for (int64_t i = threadIdx.x; i < a.L; i += blockDim.x) {
+        const double Pa = __ldcg(a.P[0] + i), Pb = __ldcg(a.P[1] + i);
+        tr += Pa * sum_q(1, i) + Pb * sum_q(0, i);
+        drop += (double)a.K * Pa * Pb;
+    }
+    if (a.L > 1) {
+#pragma unroll
+        for (int d = 16; d > 0; d >>= 1) {
+            tr += __shfl_xor_sync(0xffffffffu, tr, d);
+            drop += __shfl_xor_sync(0xffffffffu, drop, d);
+        }
+        if (lane == 0) {
+            dred[0][warp] = tr;
+            dred[1][warp] = drop;
+        }
+        __syncthreads();
+        tr = drop = 0.0;
+        for (int y = 0; y < 8; ++y) {
+            tr += dred[0][y];
+            drop += dred[1][y];
+        }
+    }
+    if (warp != 0) return;
+    tr = __shfl_sync(0xffffffffu, tr, 0);
+    drop = __shfl_sync(0xffffffffu, drop, 0);
+    oz_choose_warp(a.st, tr, __ldcg(&a.st->acc[1]), drop, a.cand, a.tol, a.margin, a.cx);
 }
 
 // =============================================================================
@@ -688,21 +839,27 @@ __device__ __forceinline__ void oz_clear_counters(int32_t *cnt, int n) {
         for (int i = threadIdx.x; i < n; i += blockDim.x) cnt[i] = 0;
 }
 
-// `sel` (nullable): the adaptive choice; the slice count is read from it and
-// the launch does nothing when it is 0 (plain).
-template <typename T, int MODE, bool BF3>
-__global__ void __launch_bounds__(256, 4) k_oz_slice(const T *__restrict__ X, OpGeom g,
-                                                  const int32_t *__restrict__ exps, int S,
-                                                  uint32_t *__restrict__ out, int64_t rows_e,
-                                                  int64_t kw, const int32_t *__restrict__ sel,
-                                                  int32_t *cnt, int ncnt) {
-    if (sel) {
-        S = *sel;
+// Slices of both operands (see PrePair). With an adaptive choice the slice
+// count is read from it, and the launch does nothing when it is 0 (plain).
+template <typename T, bool CX, bool BF3>
+__global__ void __launch_bounds__(256, 4) k_oz_slice(const __grid_constant__ PrePair a, int only) {
+    int S = a.S;
+    if (a.sel) {
+        S = *a.sel;
         if (S == 0) return;
     }
-    if (blockIdx.x == 0 && blockIdx.y == 0) oz_clear_counters(cnt, ncnt);
-    __shared__ SliceSmemOf<T, MODE> sm;
-    oz_slice_tile<T, MODE, BF3>(X, g, exps, S, out, rows_e, kw, blockIdx.x, blockIdx.y, sm);
+    if (blockIdx.x == 0 && blockIdx.y == 0) oz_clear_counters(a.cnt, a.ncnt);
+    __shared__ SliceSmemOf<T, MODE_REAL> sm;
+    int64_t blk;
+    if (pre_operand(a, only, blk) == 0) {
+        const PreOperand &p = a.op[0];
+        oz_slice_tile<T, CX ? MODE_CA : MODE_REAL, BF3>((const T *)p.X, p.g, p.exps, S, p.out, p.rows_e, a.kw, blk,
+                                                        blockIdx.y, sm);
+    } else {
+        const PreOperand &p = a.op[1];
+        oz_slice_tile<T, CX ? MODE_CB : MODE_REAL, BF3>((const T *)p.X, p.g, p.exps, S, p.out, p.rows_e, a.kw, blk,
+                                                        blockIdx.y, sm);
+    }
 }
 
 // =============================================================================
@@ -900,6 +1057,11 @@ static OzStatArea stat_area(const ContractionPlan &p, void *ws) {
     a.partb = (int2 *)((uint8_t *)ws + off);
     return a;
 }
+// Fluctuations of a Frobenius norm over few outputs: a margin on the estimate
+// that vanishes for large results.
+static double choice_margin(const ContractionPlan &p) {
+    return 1.0 + 2.0 / std::sqrt((double)std::max<int64_t>(p.M * p.N * p.L, 1));
+}
 static uint64_t stat_bytes(const ContractionPlan &p) {
     return align256(align256(sizeof(OzStats) + 2 * (uint64_t)p.L * 4) + 2 * (uint64_t)p.L * p.K * 4);
 }
@@ -940,42 +1102,6 @@ static int unit_row_fast(const ModeGroup &gr, const ModeGroup &gk, int t) {
     return sr <= sk ? 1 : 0;
 }
 
-template <typename T, bool BF3>
-static int run_prepass(const OpGeom &g, int mode, const void *X, int32_t *exps, int S, uint32_t *out,
-                       int64_t rows_e, int64_t kw, int64_t L, cudaStream_t s, const int32_t *sel = nullptr,
-                       int32_t *cnt = nullptr, int ncnt = 0) {
-    int64_t tiles = ((g.R + 31) / 32) * ((g.K + OZ_SLICE_KT - 1) / OZ_SLICE_KT);
-    if (tiles > INT32_MAX) return fail(MGB_ERR_UNSUPPORTED, "operand too large for the slicer grid");
-    dim3 grid((unsigned)tiles, (unsigned)L);
-    const T *x = (const T *)X;
-    switch (mode) {
-    case MODE_REAL: k_oz_slice<T, MODE_REAL, BF3><<<grid, 256, 0, s>>>(x, g, exps, S, out, rows_e, kw, sel, cnt, ncnt); break;
-    case MODE_CA: k_oz_slice<T, MODE_CA, BF3><<<grid, 256, 0, s>>>(x, g, exps, S, out, rows_e, kw, sel, cnt, ncnt); break;
-    default: k_oz_slice<T, MODE_CB, BF3><<<grid, 256, 0, s>>>(x, g, exps, S, out, rows_e, kw, sel, cnt, ncnt); break;
-    }
-    MGB_CUDA_CHECK(cudaGetLastError());
-    return MGB_OK;
-}
-
-template <typename T>
-static int run_scale(const OpGeom &g, const void *X, int32_t *exps, int64_t L, cudaStream_t s,
-                     int32_t *emax = nullptr, int2 *part = nullptr) {
-    int64_t tiles = ((g.R + 31) / 32) * ((g.K + OZ_SCAN_KT - 1) / OZ_SCAN_KT);
-    if (tiles > INT32_MAX) return fail(MGB_ERR_UNSUPPORTED, "operand too large for the scale grid");
-    dim3 grid((unsigned)tiles, (unsigned)L);
-    k_oz_scale<T><<<grid, 256, 0, s>>>((const T *)X, g, exps, emax, part);
-    MGB_CUDA_CHECK(cudaGetLastError());
-    return MGB_OK;
-}
-
-static int run_stat(const int2 *part, const int32_t *exps, OzStats *st, int t, float *q, float *P, int64_t R,
-                    int64_t K, int64_t L, cudaStream_t s) {
-    const int64_t blocks = oz_stat_blocks(R, K);
-    if (blocks > INT32_MAX) return fail(MGB_ERR_UNSUPPORTED, "operand too large for the statistics grid");
-    k_oz_stat<<<dim3((unsigned)blocks, (unsigned)L), 256, 0, s>>>(part, exps, st, t, q, P, R, K);
-    MGB_CUDA_CHECK(cudaGetLastError());
-    return MGB_OK;
-}
 // Calls f with a null pointer of the operand's element type.
 template <typename F>
 static int by_type(int dtype, F &&f) {
@@ -989,122 +1115,138 @@ static int by_type(int dtype, F &&f) {
 template <typename P>
 using TypeOf = typename std::remove_pointer<P>::type;
 
-// Pre-pass of the emulated forms: exponents (OZAKI) and slices of A and B
-// into the workspace.
+// Launches f(type tag, operand) for both operands at once (operand -1) when
+// their element types agree, else one by one.
+template <typename F>
+static int by_operand(const ContractionPlan &p, F &&f) {
+    if (p.a.dtype == p.b.dtype) return by_type(p.a.dtype, [&](auto tag) { return f(tag, -1); });
+    if (int st = by_type(p.a.dtype, [&](auto tag) { return f(tag, 0); })) return st;
+    return by_type(p.b.dtype, [&](auto tag) { return f(tag, 1); });
+}
+
+// Pre-pass of the emulated forms into the workspace: exponents, for adaptive
+// plans the statistics and the choice (OZAKI), and slices of A and B. One
+// launch per phase.
 int ozaki_prepass(const ContractionPlan &p, const void *A, const void *B, void *ws, bool split, cudaStream_t s) {
     if (((uintptr_t)ws & 255) != 0) return fail(MGB_ERR_WORKSPACE, "workspace must be 256-byte aligned");
     const bool exact = p.form == MGB_FORM_OZAKI;
     const bool cx = is_complex(p.compute_dtype);
-    const int S = p.slices;
     uint8_t *w = (uint8_t *)ws;
-    uint32_t *sa = (uint32_t *)(w + p.ws_a), *sb = (uint32_t *)(w + p.ws_b);
-    int32_t *ea = exact ? (int32_t *)(w + p.ws_scale_a) : nullptr;
-    int32_t *eb = exact ? (int32_t *)(w + p.ws_scale_b) : nullptr;
+    OzStatArea area = {};
+    if (exact && p.adaptive) area = stat_area(p, ws);
 
-    OpGeom ga, gb;
-    ga.ptrs = p.pa;
-    gb.ptrs = p.pb;
-    ga.gr = p.gm; ga.gk = p.gk; ga.gl = p.gl; ga.t = 0; ga.R = p.M; ga.K = p.K;
-    ga.rows_fast = unit_row_fast(p.gm, p.gk, 0);
-    gb.gr = p.gn; gb.gk = p.gk; gb.gl = p.gl; gb.t = 1; gb.R = p.N; gb.K = p.K;
-    gb.rows_fast = unit_row_fast(p.gn, p.gk, 1);
-    const int64_t kw = p.kpad / 2;
-    const int mode_a = cx ? MODE_CA : MODE_REAL, mode_b = cx ? MODE_CB : MODE_REAL;
-    int32_t *cnt = nullptr;  // counters of split tiles, cleared with the slicing of A
-    const int ncnt = split ? split_counters(p) : 0;
-    if (ncnt) cnt = (int32_t *)(w + p.ws_cnt);
-    int st;
-    if (exact) {
-        MGB_CUDA_CHECK(cudaMemsetAsync(ea, 0, (size_t)p.L * p.M * 4, s));
-        MGB_CUDA_CHECK(cudaMemsetAsync(eb, 0, (size_t)p.L * p.N * 4, s));
-        OzStatArea sa_ = {};
-        const int32_t *sel = nullptr;
-        if (p.adaptive) {
-            sa_ = stat_area(p, ws);
-            MGB_CUDA_CHECK(cudaMemsetAsync(sa_.st, 0, stat_bytes(p), s));
-            sel = &sa_.st->sel;
-        }
-        int32_t *emax_a = p.adaptive ? &sa_.st->emax[0] : nullptr, *emax_b = p.adaptive ? &sa_.st->emax[1] : nullptr;
-        st = by_type(p.a.dtype,
-                     [&](auto tag) { return run_scale<TypeOf<decltype(tag)>>(ga, A, ea, p.L, s, emax_a, sa_.parta); });
-        if (st) return st;
-        st = by_type(p.b.dtype,
-                     [&](auto tag) { return run_scale<TypeOf<decltype(tag)>>(gb, B, eb, p.L, s, emax_b, sa_.partb); });
-        if (st) return st;
-        if (p.adaptive) {
-            if ((st = run_stat(sa_.parta, ea, sa_.st, 0, sa_.qa, sa_.pa, p.M, p.K, p.L, s))) return st;
-            if ((st = run_stat(sa_.partb, eb, sa_.st, 1, sa_.qb, sa_.pb, p.N, p.K, p.L, s))) return st;
-            // Fluctuations of a Frobenius norm over few outputs: a margin that
-            // vanishes for large results.
-            const double margin = 1.0 + 2.0 / std::sqrt((double)std::max<int64_t>(p.M * p.N * p.L, 1));
-            const int64_t eb = oz_est_blocks(p.K) * p.L;
-            if (eb > INT32_MAX) return fail(MGB_ERR_UNSUPPORTED, "operand too large for the estimate grid");
-            k_oz_est<<<(unsigned)eb, 256, 0, s>>>(sa_.st, sa_.qa, sa_.qb, sa_.pa, sa_.pb, p.K);
-            MGB_CUDA_CHECK(cudaGetLastError());
-            k_oz_choose<<<1, 32, 0, s>>>(sa_.st, p.cand_mask, p.tol, margin, cx ? 1 : 0);
-            MGB_CUDA_CHECK(cudaGetLastError());
-        }
-        st = by_type(p.a.dtype, [&](auto tag) {
-            return run_prepass<TypeOf<decltype(tag)>, false>(ga, mode_a, A, ea, S, sa, p.m_e, kw, p.L, s, sel, cnt, ncnt);
-        });
-        if (st) return st;
-        st = by_type(p.b.dtype, [&](auto tag) {
-            return run_prepass<TypeOf<decltype(tag)>, false>(gb, mode_b, B, eb, S, sb, p.n_e, kw, p.L, s, sel);
-        });
-        if (st) return st;
-    } else {
-        st = p.a.dtype == MGB_C32 ? run_prepass<float2, true>(ga, mode_a, A, nullptr, 3, sa, p.m_e, kw, p.L, s, nullptr,
-                                                              cnt, ncnt)
-                                  : run_prepass<float, true>(ga, mode_a, A, nullptr, 3, sa, p.m_e, kw, p.L, s, nullptr,
-                                                             cnt, ncnt);
-        if (st) return st;
-        st = p.b.dtype == MGB_C32 ? run_prepass<float2, true>(gb, mode_b, B, nullptr, 3, sb, p.n_e, kw, p.L, s)
-                                  : run_prepass<float, true>(gb, mode_b, B, nullptr, 3, sb, p.n_e, kw, p.L, s);
-        if (st) return st;
+    PrePair pre;
+    for (int o = 0; o < 2; ++o) {
+        PreOperand &q = pre.op[o];
+        q.g.gr = o ? p.gn : p.gm;
+        q.g.gk = p.gk;
+        q.g.gl = p.gl;
+        q.g.ptrs = o ? p.pb : p.pa;
+        q.g.t = o;
+        q.g.R = o ? p.N : p.M;
+        q.g.K = p.K;
+        q.g.rows_fast = unit_row_fast(q.g.gr, p.gk, o);
+        q.X = o ? B : A;
+        q.exps = exact ? (int32_t *)(w + (o ? p.ws_scale_b : p.ws_scale_a)) : nullptr;
+        q.part = o ? area.partb : area.parta;
+        q.out = (uint32_t *)(w + (o ? p.ws_b : p.ws_a));
+        q.rows_e = o ? p.n_e : p.m_e;
+        static_assert(OZ_SCAN_KT == OZ_SLICE_KT, "the scan and the slicer walk the same tiles");
+        q.tiles = ((q.g.R + 31) / 32) * ((p.K + OZ_SLICE_KT - 1) / OZ_SLICE_KT);
     }
-    return MGB_OK;
+    if (pre.op[0].tiles + pre.op[1].tiles > INT32_MAX)
+        return fail(MGB_ERR_UNSUPPORTED, "operand too large for the slicer grid");
+    pre.emax = area.st ? area.st->emax : nullptr;
+    pre.kw = p.kpad / 2;
+    pre.sel = area.st ? &area.st->sel : nullptr;
+    pre.S = exact ? p.slices : 3;
+    pre.ncnt = split ? split_counters(p) : 0;
+    pre.cnt = pre.ncnt ? (int32_t *)(w + p.ws_cnt) : nullptr;
+    auto grid = [&](int o) {
+        return dim3((unsigned)(o < 0 ? pre.op[0].tiles + pre.op[1].tiles : pre.op[o].tiles), (unsigned)p.L);
+    };
+    if (exact) {
+        // exponents, statistics header and sums: one contiguous area
+        uint64_t end = p.ws_scale_b + (uint64_t)p.L * p.N * 4;
+        if (p.adaptive)
+            end = p.K > 1 ? (uint64_t)((uint8_t *)area.qa - w) + 2 * (uint64_t)p.L * sizeof(double)
+                          : (uint64_t)((uint8_t *)(area.pb + p.L) - w);
+        MGB_CUDA_CHECK(cudaMemsetAsync(w + p.ws_scale_a, 0, end - p.ws_scale_a, s));
+        int st = by_operand(p, [&](auto tag, int o) -> int {
+            k_oz_scale<TypeOf<decltype(tag)>><<<grid(o), 256, 0, s>>>(pre, o);
+            MGB_CUDA_CHECK(cudaGetLastError());
+            return MGB_OK;
+        });
+        if (st) return st;
+        if (p.adaptive) {
+            StatArgs a;
+            a.part[0] = area.parta;
+            a.part[1] = area.partb;
+            a.exps[0] = pre.op[0].exps;
+            a.exps[1] = pre.op[1].exps;
+            a.R[0] = p.M;
+            a.R[1] = p.N;
+            a.K = p.K;
+            a.L = p.L;
+            a.st = area.st;
+            a.P[0] = area.pa;
+            a.P[1] = area.pb;
+            a.Q[0] = area.qa;
+            a.Q[1] = p.K > 1 ? (void *)((double *)area.qa + p.L) : (void *)(area.qa + p.L);
+            a.tol = p.tol;
+            a.margin = choice_margin(p);
+            a.cand = p.cand_mask;
+            a.cx = cx ? 1 : 0;
+            const int64_t blocks = oz_stat_grid(p.M, p.N, p.K);
+            if (blocks * p.L > INT32_MAX) return fail(MGB_ERR_UNSUPPORTED, "operand too large for the statistics grid");
+            k_oz_stat<<<dim3((unsigned)blocks, (unsigned)p.L), 256, 0, s>>>(a);
+            MGB_CUDA_CHECK(cudaGetLastError());
+        }
+    }
+    return by_operand(p, [&](auto tag, int o) -> int {
+        using T = TypeOf<decltype(tag)>;
+        if (exact) {
+            if (cx) k_oz_slice<T, true, false><<<grid(o), 256, 0, s>>>(pre, o);
+            else if constexpr (!OzIn<T>::cx) k_oz_slice<T, false, false><<<grid(o), 256, 0, s>>>(pre, o);
+        } else if constexpr (std::is_same<T, float>::value || std::is_same<T, float2>::value) {
+            if (cx) k_oz_slice<T, true, true><<<grid(o), 256, 0, s>>>(pre, o);
+            else if constexpr (!OzIn<T>::cx) k_oz_slice<T, false, true><<<grid(o), 256, 0, s>>>(pre, o);
+        }
+        MGB_CUDA_CHECK(cudaGetLastError());
+        return MGB_OK;
+    });
 }
 
-// The GEMM's view of a plan whose slices lie in `ws`.
-// `split`: the workspace has room for the sums of split tiles (ws_bytes, not only ws_min).
-static int ozaki_job(const ContractionPlan &p, void *C, void *ws, bool split, OzJob &job, int64_t &units, int S = 0,
-                     const int32_t *sel = nullptr) {
+// The GEMM's view of a plan whose slices lie in `ws`. `split`: the workspace
+// has room for the sums of split tiles (ws_bytes, not only ws_min).
+static int ozaki_shape(const ContractionPlan &p, void *C, void *ws, bool split, OzJobShape &job) {
     const bool exact = p.form == MGB_FORM_OZAKI;
-    if (S == 0) S = p.slices;
     uint8_t *w = (uint8_t *)ws;
-    uint32_t *sa = (uint32_t *)(w + p.ws_a), *sb = (uint32_t *)(w + p.ws_b);
     int32_t *status = device_status_ptr();
     if (!status) return fail(MGB_ERR_CUDA, "device status word unavailable");
-    std::memset(&job, 0, sizeof(job));
-    int st;
-    if ((st = make_map(&job.tmA, sa, p.k_e, p.m_e, p.L * S, p.kpad, OZ_BM, S))) return st;
-    const int bn = oz_bn(S, exact);
-    if ((st = make_map(&job.tmB, sb, p.k_e, p.n_e, p.L * S, p.kpad, bn, S))) return st;
+    const int bn = oz_bn(p.slices, exact);
     OzGemmArgs &a = job.a;
     a.M = p.M;
     a.Ne = p.n_e;
     a.N = p.N;
     a.nkb = (int32_t)((p.k_e + OZ_BK - 1) / OZ_BK);
-    a.kcb = exact ? oz_chunk_blocks(S) : OZ_KC / OZ_BK;
-    a.S = S;
     a.expA = exact ? (int32_t *)(w + p.ws_scale_a) : nullptr;
     a.expB = exact ? (int32_t *)(w + p.ws_scale_b) : nullptr;
     a.C = C;
     a.cptr = p.pc;
-    if (p.band > 0) {
-        a.band = p.band;
-    } else {
-        a.band = OZ_GROUP_M;
-        while (a.band > 1 && (int64_t)a.band * OZ_BM * p.kpad * S * 2 > OZ_BAND_BYTES) --a.band;
-    }
     a.gm = p.gm;
     a.gn = p.gn;
     a.gl = p.gl;
     a.status = status;
-    a.sel = sel;
+    a.sel = nullptr;
     if (a.gm.n == 0) { a.gm.n = 1; a.gm.ext[0] = 1; for (int t = 0; t < 3; ++t) a.gm.str[t][0] = 0; }
     if (a.gn.n == 0) { a.gn.n = 1; a.gn.ext[0] = 1; for (int t = 0; t < 3; ++t) a.gn.str[t][0] = 0; }
-    a.full = INT64_MAX;
+    job.tiles_n = (int32_t)((p.n_e + bn - 1) / bn);
+    job.tiles_m = (int32_t)((p.M + OZ_BM - 1) / OZ_BM);
+    job.L = (int32_t)p.L;
+    if ((p.n_e + bn - 1) / bn > INT32_MAX || (p.M + OZ_BM - 1) / OZ_BM > INT32_MAX || p.L > INT32_MAX)
+        return fail(MGB_ERR_UNSUPPORTED, "contraction too large for the tile grid");
+    a.full = (int64_t)job.tiles_n * job.tiles_m * job.L;
     a.splits = 1;
     a.kbs = a.nkb;
     if (split && p.splits > 1) {
@@ -1114,33 +1256,50 @@ static int ozaki_job(const ContractionPlan &p, void *C, void *ws, bool split, Oz
         a.cnt = (int32_t *)(w + p.ws_cnt);
         a.part = (uint32_t *)(w + p.ws_part);
     }
-    job.tiles_n = (int32_t)((p.n_e + bn - 1) / bn);
-    job.tiles_m = (int32_t)((p.M + OZ_BM - 1) / OZ_BM);
-    job.L = (int32_t)p.L;
-    if ((p.n_e + bn - 1) / bn > INT32_MAX || (p.M + OZ_BM - 1) / OZ_BM > INT32_MAX || p.L > INT32_MAX)
-        return fail(MGB_ERR_UNSUPPORTED, "contraction too large for the tile grid");
-    const int64_t all = (int64_t)job.tiles_n * job.tiles_m * job.L;
-    if (a.full > all) a.full = all;
-    units = job.units();
     return MGB_OK;
+}
+// The slice tensor maps and the band for S slices.
+static int ozaki_maps(const ContractionPlan &p, void *ws, int S, CUtensorMap *ta, CUtensorMap *tb, int32_t &band) {
+    uint8_t *w = (uint8_t *)ws;
+    int st;
+    if ((st = make_map(ta, w + p.ws_a, p.k_e, p.m_e, p.L * S, p.kpad, OZ_BM, S))) return st;
+    if ((st = make_map(tb, w + p.ws_b, p.k_e, p.n_e, p.L * S, p.kpad, oz_bn(S, p.form == MGB_FORM_OZAKI), S))) return st;
+    band = p.band;
+    if (band <= 0) {
+        band = OZ_GROUP_M;
+        while (band > 1 && (int64_t)band * OZ_BM * p.kpad * S * 2 > OZ_BAND_BYTES) --band;
+    }
+    return MGB_OK;
+}
+// A job of slice count S (0: the plan's), run only when `sel` (nullable) holds S.
+static int ozaki_job(const ContractionPlan &p, void *C, void *ws, bool split, OzJob &job, int64_t &units, int S = 0,
+                     const int32_t *sel = nullptr) {
+    std::memset(&job, 0, sizeof(job));
+    if (int st = ozaki_shape(p, C, ws, split, job)) return st;
+    job.a.sel = sel;
+    units = job.units();
+    return ozaki_maps(p, ws, S ? S : p.slices, &job.tmA, &job.tmB, job.band);
 }
 
 int ozaki_gemm(const ContractionPlan &p, const void *A, const void *B, void *C, void *ws, bool split, cudaStream_t s) {
-    int st;
-    OzJob job;
-    int64_t tiles = 0;
+    int64_t units = 0;
+    const bool cx = is_complex(p.compute_dtype);
     if (!p.adaptive) {
-        if ((st = ozaki_job(p, C, ws, split, job, tiles))) return st;
-        return oz_launch_one(p.slices, p.form == MGB_FORM_OZAKI, is_complex(p.compute_dtype), job, tiles, s);
+        OzJob job;
+        if (int st = ozaki_job(p, C, ws, split, job, units)) return st;
+        return oz_launch_one(p.slices, p.form == MGB_FORM_OZAKI, cx, job, units, s);
     }
-    // Every candidate is launched; the kernel of the chosen count works and
-    // the others return at once. With no count chosen the plain form runs.
+    // One launch, which reads the chosen count; with none chosen the plain form runs.
+    OzAnyJob job;
+    std::memset(&job, 0, sizeof(job));
+    if (int st = ozaki_shape(p, C, ws, split, job)) return st;
     const int32_t *sel = &stat_area(p, ws).st->sel;
-    for (int S = 3; S <= 8; ++S) {
-        if (!(p.cand_mask & (1u << S))) continue;
-        if ((st = ozaki_job(p, C, ws, split, job, tiles, S, sel))) return st;
-        if ((st = oz_launch_one(S, true, is_complex(p.compute_dtype), job, tiles, s))) return st;
-    }
+    job.a.sel = sel;
+    job.cand = p.cand_mask;
+    for (int S = 3; S <= 8; ++S)
+        if (p.cand_mask & (1u << S))
+            if (int st = ozaki_maps(p, ws, S, &job.tm[S - 3][0], &job.tm[S - 3][1], job.band[S - 3])) return st;
+    if (int st = oz_launch_any(cx, job, job.units(), s)) return st;
     return launch_plain_gemm(p, A, B, C, s, sel);
 }
 
@@ -1283,40 +1442,11 @@ struct ChooseJob {
     double tol, margin;
 };
 
-union PreSmem {
-    ScaleSmem scale;
-    StatSmem stat;
-    SliceSmemOf<double, MODE_REAL> s_dr;
-    SliceSmemOf<double2, MODE_CA> s_zc;
-    SliceSmemOf<double, MODE_CA> s_dc;
-    SliceSmemOf<float, MODE_REAL> s_fr;
-    SliceSmemOf<float2, MODE_CA> s_cc;
-    SliceSmemOf<float, MODE_CA> s_fc;
-};
-
-template <typename T, bool BF3>
-__device__ __forceinline__ void pre_slice_typed(const PreJob &J, int S, int64_t blk, int64_t l, PreSmem &sm) {
-    const T *X = (const T *)J.X;
-    switch (J.mode) {
-    case MODE_REAL:
-        if constexpr (!OzIn<T>::cx)
-            oz_slice_tile<T, MODE_REAL, BF3>(X, J.g, J.exps, S, J.out, J.rows_e, J.kw, blk, l,
-                                             *reinterpret_cast<SliceSmemOf<T, MODE_REAL> *>(&sm));
-        break;
-    case MODE_CA:
-        oz_slice_tile<T, MODE_CA, BF3>(X, J.g, J.exps, S, J.out, J.rows_e, J.kw, blk, l,
-                                       *reinterpret_cast<SliceSmemOf<T, MODE_CA> *>(&sm));
-        break;
-    default:
-        oz_slice_tile<T, MODE_CB, BF3>(X, J.g, J.exps, S, J.out, J.rows_e, J.kw, blk, l,
-                                       *reinterpret_cast<SliceSmemOf<T, MODE_CB> *>(&sm));
-        break;
-    }
-}
-
-__global__ void __launch_bounds__(256, 3) k_oz_pre_multi(const PreJob *__restrict__ jobs,
+// Clearing and statistics over a table of operand jobs (the scan and the
+// slicing have typed launches of their own).
+__global__ void __launch_bounds__(256) k_oz_pre_multi(const PreJob *__restrict__ jobs,
                                                          const int64_t *__restrict__ start, int njobs, int phase) {
-    __shared__ __align__(16) PreSmem sm;
+    __shared__ StatSmem sm;
     const int64_t b = blockIdx.x;
     int lo = 0, hi = njobs - 1;  // the last job whose first block is <= b
     while (lo < hi) {
@@ -1336,33 +1466,7 @@ __global__ void __launch_bounds__(256, 3) k_oz_pre_multi(const PreJob *__restric
     }
     const int64_t per_l = J.tiles[phase] / max(J.L, 1);
     const int64_t l = local / per_l, blk = local - l * per_l;
-    if (phase == PRE_SCALE) {
-        switch (J.dtype) {
-        case MGB_F64: oz_scale_tile<double>((const double *)J.X, J.g, J.exps, J.emax, J.part, blk, l, sm.scale); break;
-        case MGB_C64: oz_scale_tile<double2>((const double2 *)J.X, J.g, J.exps, J.emax, J.part, blk, l, sm.scale); break;
-        case MGB_F32: oz_scale_tile<float>((const float *)J.X, J.g, J.exps, J.emax, J.part, blk, l, sm.scale); break;
-        default: oz_scale_tile<float2>((const float2 *)J.X, J.g, J.exps, J.emax, J.part, blk, l, sm.scale); break;
-        }
-    } else if (phase == PRE_STAT) {
-        oz_stat_block(J.part, J.exps, J.st, J.t, J.q, J.P, J.g.R, J.g.K, blk, l, sm.stat);
-    } else {
-        int S = J.S;
-        if (J.sel) {
-            S = *J.sel;
-            if (S == 0) return;  // the plain form will run this contraction
-        }
-        if (J.bf3) {
-            if (J.dtype == MGB_C32) pre_slice_typed<float2, true>(J, 3, blk, l, sm);
-            else pre_slice_typed<float, true>(J, 3, blk, l, sm);
-        } else {
-            switch (J.dtype) {
-            case MGB_F64: pre_slice_typed<double, false>(J, S, blk, l, sm); break;
-            case MGB_C64: pre_slice_typed<double2, false>(J, S, blk, l, sm); break;
-            case MGB_F32: pre_slice_typed<float, false>(J, S, blk, l, sm); break;
-            default: pre_slice_typed<float2, false>(J, S, blk, l, sm); break;
-            }
-        }
-    }
+    oz_stat_block(J.part, J.exps, J.st, J.t, J.q, J.P, J.g.R, J.g.K, blk, l, sm);
 }
 
 // dst[i] = *src[i]: every item's slice count after the choice
@@ -1434,10 +1538,12 @@ __global__ void __launch_bounds__(256) k_oz_est_multi(const ChooseJob *__restric
     const int64_t local = b - start[lo], nb = oz_est_blocks(c.K), l = local / nb;
     oz_est_block(c.st, c.qa, c.qb, c.pa, c.pb, c.K, local - l * nb, l, red);
 }
-// One thread per adaptive contraction: its estimate and choice.
+// One warp per adaptive contraction: its estimate and choice.
 __global__ void k_oz_choose_multi(const ChooseJob *__restrict__ jobs, int njobs) {
-    const int j = blockIdx.x * blockDim.x + threadIdx.x;
-    if (j < njobs) oz_choose_final(jobs[j].st, jobs[j].cand, jobs[j].tol, jobs[j].margin, jobs[j].cx);
+    const int j = (blockIdx.x * blockDim.x + threadIdx.x) / 32;
+    if (j >= njobs) return;
+    const ChooseJob &c = jobs[j];
+    oz_choose_warp(c.st, c.st->acc[0], c.st->acc[1], c.st->acc[2], c.cand, c.tol, c.margin, c.cx);
 }
 
 struct OzBatchBuffers {
@@ -1541,7 +1647,7 @@ static ChooseJob choose_job(const ContractionPlan &p, void *ws) {
     c.cand = p.cand_mask;
     c.cx = is_complex(p.compute_dtype) ? 1 : 0;
     c.tol = p.tol;
-    c.margin = 1.0 + 2.0 / std::sqrt((double)std::max<int64_t>(p.M * p.N * p.L, 1));
+    c.margin = choice_margin(p);
     return c;
 }
 
@@ -1693,7 +1799,7 @@ static int pre_launch(const PreLayout &L, size_t npre, size_t nch, const uint8_t
                                                                       (const int64_t *)(d + L.o_cs), (int)nch);
                 MGB_CUDA_CHECK(cudaGetLastError());
             }
-            k_oz_choose_multi<<<((int)nch + 127) / 128, 128, 0, s>>>((const ChooseJob *)(d + L.o_ch), (int)nch);
+            k_oz_choose_multi<<<((int)nch + 3) / 4, 128, 0, s>>>((const ChooseJob *)(d + L.o_ch), (int)nch);
             MGB_CUDA_CHECK(cudaGetLastError());
         }
         if (ph == PRE_SCALE || ph == PRE_SLICE) {
