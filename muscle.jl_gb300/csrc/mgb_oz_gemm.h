@@ -148,11 +148,14 @@ __device__ __forceinline__ uint64_t sw64_desc(uint32_t saddr) {
     d |= (uint64_t)4 << 61;                   // swizzle mode: 64 B
     return d;
 }
-// kind::f16 instruction descriptor: f32 accumulate, bf16 A and B, both
-// K-major, M = 128, N = n (a multiple of 16 up to 256).
-__host__ __device__ constexpr uint32_t oz_idesc(int n) {
-    return (1u << 4) | (1u << 7) | (1u << 10) | ((uint32_t)(n >> 3) << 17) | ((uint32_t)(OZ_BM >> 4) << 24);
+// kind::f16 instruction descriptor: f32 accumulate, Float16 digits (EXACT) or
+// bf16 pieces for both A and B, both K-major, M = 128, N = n (a multiple of 16
+// up to 256).
+__host__ __device__ constexpr uint32_t oz_idesc(int n, bool exact) {
+    const uint32_t type = exact ? 0u : 1u;
+    return (1u << 4) | (type << 7) | (type << 10) | ((uint32_t)(n >> 3) << 17) | ((uint32_t)(OZ_BM >> 4) << 24);
 }
+
 // =============================================================================
 // The tcgen05 GEMM over slices
 // =============================================================================
@@ -541,7 +544,7 @@ __device__ __forceinline__ void oz_gemm_body(const Src &src) {
 #pragma unroll
                             for (int i = 0; i < S; ++i)
                                 tc_mma(d0 + BN * i, ad0 + (uint64_t)((i * OZ_A_TILE + k16 * 32) >> 4),
-                                       bd0 + (uint64_t)((k16 * 32) >> 4), oz_idesc(BN * (S - i)), 1u);
+                                       bd0 + (uint64_t)((k16 * 32) >> 4), oz_idesc(BN * (S - i), EXACT), 1u);
                         tc_commit(smem_u32(empty + s));
                     }
                     if (ok) tc_commit(smem_u32(acc_full + bank));

@@ -5,7 +5,7 @@
 //   largest exponent; the scaled value a in [-1, 1] is cut into S signed
 //   W-bit digits by round-to-nearest:  a = sum_i s_i 2^(-W i) + r,
 //   |s_1| <= 2^W, |s_i| <= 2^(W-1), |r| <= 2^(-W S - 1).  W = 8 for S <= 6
-//   and W = 7 for S >= 7: every digit is an integer that bf16 holds exactly,
+//   and W = 7 for S >= 7: every digit is an integer that Float16 holds exactly,
 //   every digit product is exact, and a float32 accumulator stays exact
 //   while the sum of the absolute products it receives is <= 2^24.
 //   Products s_i t_j with i + j = d share the scale 2^(-W d) and go to one
@@ -54,6 +54,7 @@
 // MMAs, frees TMEM and returns.
 #include <cuda.h>
 #include <cuda_bf16.h>
+#include <cuda_fp16.h>
 
 #include <algorithm>
 #include <atomic>
@@ -81,11 +82,11 @@ struct OpGeom {
     int t;                 // tensor index inside the groups (0 = A, 1 = B)
     int64_t R, K;
     int rows_fast;         // operand's unit-stride mode is a row mode
+    int scan_lk;           // exponent scan: log2 of a block's warps along k
+    int kvec;              // 16-byte vectors along k are aligned, if the base is
 };
 
-__device__ __forceinline__ int bexp(double v) {
-    return (int)((__double_as_longlong(v) >> 52) & 0x7FF);
-}
+__device__ __forceinline__ int bexp(double v) { return (__double2hiint(v) >> 20) & 0x7FF; }
 __device__ __forceinline__ int bexp_of(double v) { return bexp(v); }
 __device__ __forceinline__ int bexp_of(double2 v) { return max(bexp(v.x), bexp(v.y)); }
 // Float32 operands of a Float64 / ComplexF64 contraction (promote_eltype),
@@ -93,141 +94,130 @@ __device__ __forceinline__ int bexp_of(double2 v) { return max(bexp(v.x), bexp(v
 __device__ __forceinline__ int bexp_of(float v) { return bexp((double)v); }
 __device__ __forceinline__ int bexp_of(float2 v) { return max(bexp((double)v.x), bexp((double)v.y)); }
 
-// `emax` (nullable): also the largest exponent of the whole operand.
 // 2^(2 d) as a float (0 below 2^-126)
 __device__ __forceinline__ float pow4f(int d) { return d >= -63 ? __int_as_float((127 + 2 * d) << 23) : 0.f; }
-
-// k per tile of the exponent scan: each thread issues eight loads before
-// the first reduction.
-constexpr int OZ_SCAN_KT = 64;
-
-struct ScaleSmem {
-    int64_t roff[32], koff[OZ_SCAN_KT];
-    int red[8][33];
-    int cmax[8][OZ_SCAN_KT + 1];    // partials: per-warp column maxima
-    float csum[8][OZ_SCAN_KT + 1];  // partials: per-warp column sums
-    int tmax[OZ_SCAN_KT];           // partials: column maxima over the tile
-};
-
 // |x|^2 4^-(t - 1023), from the exponent and the top of the mantissa, for an
 // element whose biased exponent is at most t (zero, subnormal and non-finite
 // elements give 0: negligible, or flagged through the exponent table)
 __device__ __forceinline__ float sq_tile(double x, int t) {
-    const uint64_t b = (uint64_t)__double_as_longlong(x);
-    const int be = (int)((b >> 52) & 0x7FF);
-    if (be == 0 || be == 0x7FF) return 0.f;
-    const float f = __int_as_float(0x3F800000 | (uint32_t)((b >> 29) & 0x7FFFFF));
-    return f * f * pow4f(be - t);
+    const uint32_t h = (uint32_t)__double2hiint(x);
+    const int be = (int)((h >> 20) & 0x7FF);
+    const float f = __uint_as_float(0x3F800000u | (__funnelshift_l((uint32_t)__double2loint(x), h, 3) & 0x7FFFFFu));
+    return (be == 0 || be == 0x7FF) ? 0.f : f * f * pow4f(be - t);
 }
 __device__ __forceinline__ float sq_tile(double2 x, int t) { return sq_tile(x.x, t) + sq_tile(x.y, t); }
 __device__ __forceinline__ float sq_tile(float x, int t) { return sq_tile((double)x, t); }
 __device__ __forceinline__ float sq_tile(float2 x, int t) { return sq_tile((double)x.x, t) + sq_tile((double)x.y, t); }
+
+// Exponent scan. A warp takes 32 rows x 32 k with one lane per k (rows_fast:
+// per row) and four or eight loads in flight, so that one of the two reductions stays
+// in registers and the other is one warp instruction (redux) per row (per k).
+// A block is 2^(3 - lk) row tiles by 2^lk k tiles of its eight warps (wide in
+// k, for the row maxima meet in shared memory before they go to the table).
+// The integer ALU bounds it: 69 instructions per Float64 element with shuffles
+// and shared-memory column sums, about 25 now.
+constexpr int OZ_SCAN_WARPS = 8;
+struct ScaleSmem {
+    int64_t roff[32 * OZ_SCAN_WARPS], koff[32 * OZ_SCAN_WARPS];
+    int red[OZ_SCAN_WARPS][33];
+};
+__host__ __device__ inline int64_t oz_scan_tiles(int64_t R, int64_t K, int lk) {
+    const int64_t rb = 32ll << (3 - lk), kb = 32ll << lk;
+    return ((R + rb - 1) / rb) * ((K + kb - 1) / kb);
+}
+// Warps along k: as many as K fills
+static int oz_scan_lk(int64_t K) { return K > 128 ? 3 : K > 64 ? 2 : K > 32 ? 1 : 0; }
+
+// `part` (nullable, adaptive plans): per 32-row tile and k, the tile's largest
+// exponent t and the sum of |x|^2 4^-(t - 1023) over its rows, at
+// part[(l * ceil(R / 32) + tile) * K + k]. `emax` (nullable): the largest
+// exponent of the whole operand.
 template <typename T>
-// One 32-row x 64-k tile. `part` (nullable, adaptive plans): per 32-row tile
-// and k, the tile's largest exponent t and the sum of |x|^2 4^-(t - 1023)
-// over its rows, at part[(l * ceil(R / 32) + tile) * K + k].
 __device__ __forceinline__ void oz_scale_tile(const T *__restrict__ X, const OpGeom &g, int32_t *exps,
                                               int32_t *emax, int2 *part, int64_t blk, int64_t l, ScaleSmem &sm) {
-    constexpr int KT = OZ_SCAN_KT;
-    int64_t tiles_k = (g.K + KT - 1) / KT;
-    int64_t tr = blk / tiles_k, tk = blk - tr * tiles_k;
-    int64_t r0 = tr * 32, k0 = tk * KT;
-    int tid = threadIdx.x, tx = tid % 32, ty = tid / 32;
-    if (tid < 32) sm.roff[tid] = (r0 + tid < g.R) ? group_offset(g.gr, g.t, r0 + tid) : 0;
-    else if (tid < 32 + KT) sm.koff[tid - 32] = (k0 + tid - 32 < g.K) ? group_offset(g.gk, g.t, k0 + tid - 32) : 0;
+    const int lk = g.scan_lk, wk = 1 << lk;
+    const int64_t tiles_k = (g.K + (32 << lk) - 1) / (32 << lk);
+    const int64_t tr = blk / tiles_k, tk = blk - tr * tiles_k;
+    const int64_t R0 = tr * (32 << (3 - lk)), K0 = tk * (32 << lk);
+    const int tid = threadIdx.x, lane = tid % 32, warp = tid / 32;
+    if (tid < (32 << (3 - lk))) sm.roff[tid] = (R0 + tid < g.R) ? group_offset(g.gr, g.t, R0 + tid) : 0;
+    if (tid < (32 << lk)) sm.koff[tid] = (K0 + tid < g.K) ? group_offset(g.gk, g.t, K0 + tid) : 0;
     const T *Xl = g.ptrs ? (const T *)g.ptrs[l] : X + group_offset(g.gl, g.t, l);
     __syncthreads();
-    const int64_t R32 = (g.R + 31) / 32;
-    int2 *pt = part ? part + (l * R32 + tr) * g.K + k0 : nullptr;  // this tile's partials
-    if (g.rows_fast) {  // lanes walk rows; thread column kk = ty + 8 j
-        constexpr int NJ = KT / 8;
-        const bool rin = r0 + tx < g.R;
-        T v[NJ];
+    const int rt = warp >> lk, kt = warp & (wk - 1);  // this warp's tile in the block
+    const int64_t r0 = R0 + 32 * rt, k0 = K0 + 32 * kt;
+    const int64_t *roff = sm.roff + 32 * rt, *koff = sm.koff + 32 * kt;
+    const int nr = (int)min((int64_t)32, g.R - r0), nk = (int)min((int64_t)32, g.K - k0);  // may be <= 0
+    int rmax = 0;  // largest exponent of row `lane`
+    if (nr > 0 && nk > 0) {
+        int t = 0;      // column `lane`: largest exponent
+        float q = 0.f;  // and sum of |x|^2 4^-(t - 1023)
+        constexpr int U = sizeof(T) == 16 ? 4 : 8;  // loads in flight per lane
+        if (g.rows_fast) {
+            const T *x = Xl + roff[lane];
+#pragma unroll 1
+            for (int j0 = 0; j0 < nk; j0 += U) {
+                T v[U];
 #pragma unroll
-        for (int j = 0; j < NJ; ++j) {
-            memset(&v[j], 0, sizeof(T));
-            if (rin && k0 + ty + 8 * j < g.K) v[j] = __ldg(Xl + sm.roff[tx] + sm.koff[ty + 8 * j]);
-        }
-        int e = 0;
+                for (int j = 0; j < U; ++j) {
+                    memset(&v[j], 0, sizeof(T));
+                    if (lane < nr && j0 + j < nk) v[j] = __ldg(x + koff[j0 + j]);
+                }
 #pragma unroll
-        for (int j = 0; j < NJ; ++j) {
-            const int be = bexp_of(v[j]);  // zero-filled outside the operand: 0
-            e = max(e, be);
-            if (pt) {
-                int t = be;
-#pragma unroll
-                for (int d = 16; d > 0; d >>= 1) t = max(t, __shfl_xor_sync(0xffffffffu, t, d));
-                float q = sq_tile(v[j], t);
-#pragma unroll
-                for (int d = 16; d > 0; d >>= 1) q += __shfl_xor_sync(0xffffffffu, q, d);
-                if (tx == 0 && k0 + ty + 8 * j < g.K) pt[ty + 8 * j] = make_int2(t, __float_as_int(q));
+                for (int j = 0; j < U; ++j) {
+                    const int be = bexp_of(v[j]);
+                    rmax = max(rmax, be);
+                    if (part) {
+                        // the sum over the lanes as an integer: terms are below 8,
+                        // so 32 of them stay below 2^32 in units of 2^-23
+                        const int tm = __reduce_max_sync(0xffffffffu, be);
+                        const uint32_t u = __reduce_add_sync(0xffffffffu, __float2uint_rn(sq_tile(v[j], tm) * 8388608.f));
+                        if (lane == j0 + j) {
+                            t = tm;
+                            q = (float)u * 1.1920928955078125e-7f;
+                        }
+                    }
+                }
             }
-        }
-        sm.red[ty][tx] = e;
-    } else {  // lanes walk k: columns tx and tx + 32, rows ty + 8 j
-        T v[4][2];
-        int be[4][2];
+        } else {
+            const T *x = Xl + koff[lane];
+#pragma unroll 1
+            for (int j0 = 0; j0 < nr; j0 += U) {
+                T v[U];
+                int tn = t;
 #pragma unroll
-        for (int j = 0; j < 4; ++j)
+                for (int j = 0; j < U; ++j) {
+                    memset(&v[j], 0, sizeof(T));
+                    if (lane < nk && j0 + j < nr) v[j] = __ldg(x + roff[j0 + j]);
+                }
 #pragma unroll
-            for (int h = 0; h < 2; ++h) {
-                memset(&v[j][h], 0, sizeof(T));
-                if (r0 + ty + 8 * j < g.R && k0 + tx + 32 * h < g.K)
-                    v[j][h] = __ldg(Xl + sm.roff[ty + 8 * j] + sm.koff[tx + 32 * h]);
-            }
+                for (int j = 0; j < U; ++j) {
+                    const int be = bexp_of(v[j]);
+                    tn = max(tn, be);
+                    const int m = __reduce_max_sync(0xffffffffu, be);
+                    if (lane == j0 + j) rmax = m;
+                }
+                if (part) {
+                    q *= pow4f(t - tn);
 #pragma unroll
-        for (int j = 0; j < 4; ++j) {
-            be[j][0] = bexp_of(v[j][0]);
-            be[j][1] = bexp_of(v[j][1]);
-            int e = max(be[j][0], be[j][1]);
-#pragma unroll
-            for (int d = 16; d > 0; d >>= 1) e = max(e, __shfl_xor_sync(0xffffffffu, e, d));
-            if (tx == 0) sm.red[j][ty + 8 * j] = e;  // rows ty + 8 j are distinct per (ty, j)
-        }
-        if (pt) {
-#pragma unroll
-            for (int h = 0; h < 2; ++h)
-                sm.cmax[ty][tx + 32 * h] = max(max(be[0][h], be[1][h]), max(be[2][h], be[3][h]));
-            __syncthreads();
-#pragma unroll
-            for (int h = 0; h < 2; ++h) {
-                int t = 0;
-#pragma unroll
-                for (int y = 0; y < 8; ++y) t = max(t, sm.cmax[y][tx + 32 * h]);
-                float q = 0.f;
-#pragma unroll
-                for (int j = 0; j < 4; ++j)
-                    if (be[j][h] > 0) q += sq_tile(v[j][h], t);
-                sm.csum[ty][tx + 32 * h] = q;
-                if (ty == 0) sm.tmax[tx + 32 * h] = t;
-            }
-            __syncthreads();
-            if (ty < 2) {
-                const int c = tx + 32 * ty;
-                if (k0 + c < g.K) {
-                    float s2 = 0.f;
-#pragma unroll
-                    for (int y = 0; y < 8; ++y) s2 += sm.csum[y][c];
-                    pt[c] = make_int2(sm.tmax[c], __float_as_int(s2));
+                    for (int j = 0; j < U; ++j) q += sq_tile(v[j], tn);
+                    t = tn;
                 }
             }
         }
-    }
-    __syncthreads();
-    if (tid < 32) {
-        int e = 0;
-        if (r0 + tid < g.R) {
-            if (g.rows_fast) {
-                for (int j = 0; j < 8; ++j) e = max(e, sm.red[j][tid]);
-            } else {
-                e = sm.red[tid / 8 % 4][tid];  // written by ty = tid % 8, j = tid / 8
-            }
-            if (e > 0) atomicMax(exps + l * g.R + r0 + tid, e);
+        if (part && lane < nk) {
+            const int64_t R32 = (g.R + 31) / 32;
+            part[(l * R32 + r0 / 32) * g.K + k0 + lane] = make_int2(t, __float_as_int(q));
         }
+    }
+    sm.red[warp][lane] = rmax;
+    __syncthreads();
+    if (kt == 0 && nr > 0) {
+        for (int w = 1; w < wk; ++w) rmax = max(rmax, sm.red[warp + w][lane]);
+        if (lane < nr && rmax > 0) atomicMax(exps + l * g.R + r0 + lane, rmax);
         if (emax) {
-#pragma unroll
-            for (int d = 16; d > 0; d >>= 1) e = max(e, __shfl_xor_sync(0xffffffffu, e, d));
-            if (tid == 0 && e > 0) atomicMax(emax, e);
+            const int m = __reduce_max_sync(0xffffffffu, rmax);
+            if (lane == 0 && m > 0) atomicMax(emax, m);
         }
     }
 }
@@ -244,7 +234,7 @@ struct PreOperand {
     int2 *part;         // the exponent scan's partials (adaptive) or null
     uint32_t *out;      // slice planes
     int64_t rows_e;
-    int64_t tiles;      // 32-row x 64-k tiles per batch entry
+    int64_t tiles;      // blocks per batch entry of this launch
 };
 struct OzStats;
 struct PrePair {
@@ -558,67 +548,58 @@ __global__ void __launch_bounds__(256) k_oz_stat(const __grid_constant__ StatArg
 //   MODE_CB   : rows 2r, 2r+1,  word k holds (re, -im), (im, re) (B side)
 enum { MODE_REAL = 0, MODE_CA = 1, MODE_CB = 2 };
 
-__device__ __forceinline__ uint32_t bf16_bits_of_int(int d) {
-    float f = __int_as_float(0x4B400000 + d) - 12582912.0f;  // exact for |d| < 2^22
-    return __float_as_uint(f) >> 16;                         // exact in bf16 for |d| <= 256
-}
-__device__ __forceinline__ uint32_t pack2(uint32_t lo, uint32_t hi) { return lo | (hi << 16); }
-
-// x * 2^(62 - e) truncated to a signed 62-bit fixed-point integer (|x| < 2^e).
-__device__ __forceinline__ int64_t oz_fixed(double x, int e) {
-    const uint64_t b = (uint64_t)__double_as_longlong(x);
-    const int be = (int)((b >> 52) & 0x7FF);
-    int64_t m = (int64_t)(b & 0xFFFFFFFFFFFFFull);
-    int ex;
-    if (be) {
-        m |= (int64_t)1 << 52;
-        ex = be - 1075;
-    } else {
-        ex = -1074;
-    }
-    const int sh = ex + 62 - e;  // Q = m * 2^sh < 2^62
-    int64_t Q;
-    if (sh >= 0) Q = m << sh;
-    else if (sh > -63) Q = m >> (-sh);
-    else Q = 0;
-    return (b >> 63) ? -Q : Q;
-}
-// Signed digits of Q, most significant first, rounded to nearest (balanced):
-// with B = half a unit of the last digit plus 2^(W-1) at every digit position
-// after the first, digit s >= 1 is the W-bit window of Q + B at its position
-// minus 2^(W-1), and the leading digit is everything above its position
-// (signed). |d_0| <= 2^W, |d_s| <= 2^(W-1), and the remainder below the last
-// digit lies in [-1/2, 1/2) units of it: the rounding of taking the digits
-// one at a time, with one 64-bit add for all of them instead of an add, a
-// shift and a subtract per digit.
-__host__ __device__ constexpr int64_t oz_digit_bias(int S, int W) {
-    int64_t b = (int64_t)1 << (62 - W * S - 1);
-    for (int s = 1; s < S; ++s) b += (int64_t)1 << (62 - W * (s + 1) + W - 1);
+// Signed digits of Q = x 2^(62 - e) truncated to 62 bits, most significant
+// first, rounded to nearest (balanced): with B = half a unit of the last digit
+// plus 2^(W-1) at every digit position after the first, digit s >= 1 is the
+// W-bit window of Q + B at its position minus 2^(W-1), and the leading digit
+// is everything above its position (signed). |d_0| <= 2^W, |d_s| <= 2^(W-1),
+// and the remainder below the last digit lies in [-1/2, 1/2) units of it: the
+// rounding of taking the digits one at a time, with one 64-bit add for all of
+// them. 2^62 more makes the leading digit's window d_0 + 2^W, not negative.
+__host__ __device__ constexpr uint64_t oz_digit_bias(int S, int W) {
+    uint64_t b = (1ull << 62) + (1ull << (62 - W * S - 1));
+    for (int s = 1; s < S; ++s) b += 1ull << (62 - W * (s + 1) + W - 1);
     return b;
 }
-// Digit s of a biased value Qb (Q + oz_digit_bias) as an exact float. The
-// leading digit (signed, |d| <= 2^W) goes through 1.5 * 2^23 + d; a later
-// digit's W-bit window u becomes the mantissa of 2^23 + u, from which
-// 2^23 + 2^(W-1) is subtracted: a funnel shift, a mask-and-or and one add,
-// with no integer-to-float conversion. NEG gives -d (+0 for d = 0, as d).
-template <int W, int s, bool NEG = false>
-__device__ __forceinline__ float oz_digit_f(int64_t Qb) {
-    constexpr int sh = 62 - W * (s + 1);
-    if constexpr (s == 0) {
-        const float m = __int_as_float(0x4B400000 + (int)(Qb >> sh));
-        return NEG ? 12582912.0f - m : m - 12582912.0f;
-    } else {
-        constexpr float c = 8388608.0f + (float)(1 << (W - 1));
-        const float m = __uint_as_float(0x4B000000u | ((uint32_t)((uint64_t)Qb >> sh) & ((1u << W) - 1u)));
-        return NEG ? c - m : m - c;
-    }
+// Q + B for a value of a row whose largest biased exponent is rowc - 1 (rowc
+// 10000: a row with Inf or NaN, all of whose digits are zero). The mantissa,
+// left-justified by 10, moves right by the distance to the row's exponent plus
+// one (subnormal elements have the exponent of the smallest normal one).
+__device__ __forceinline__ uint64_t oz_biased(double x, int rowc, uint64_t bias) {
+    const uint32_t lo = (uint32_t)__double2loint(x), hi = (uint32_t)__double2hiint(x);
+    const int be = (int)((hi >> 20) & 0x7FF);
+    const uint32_t mh = (hi & 0xFFFFFu) | (be ? 0x100000u : 0u);
+    const uint64_t m = ((uint64_t)__funnelshift_l(lo, mh, 10) << 32) | (lo << 10);
+    const uint64_t M = m >> min(rowc - max(be, 1), 63);
+    const uint64_t neg = (uint64_t)((int64_t)(int32_t)hi >> 63);
+    return (M ^ neg) + (bias | (hi >> 31));  // the bias is even: -M = ~M + 1
 }
-// Two floats that bf16 holds exactly (the digits: integers of at most 8
-// significant bits) as one packed word, `lo` in the low half. Their bf16
-// bits are the upper halves of their float bits, so one byte permute on the
-// integer pipe packs them (no conversion instruction).
-__device__ __forceinline__ uint32_t pack_bf16x2(float lo, float hi) {
-    return __byte_perm(__float_as_uint(lo), __float_as_uint(hi), 0x7632);
+// Digit s of two biased values as two Float16 (exact: integers up to 256),
+// the first in the low half. The windows become the low bits of 1024 + u, from
+// which 1024 and the window's offset are subtracted, both at once. For W = 8
+// the windows after the first are bytes of the values shifted left by 2 (which
+// is what the caller passes for s > 0), so a byte permute gathers both: 3
+// instructions per digit pair.
+template <int W, int s>
+__device__ __forceinline__ uint32_t oz_digit_pair(uint64_t u0, uint64_t u1) {
+    uint32_t w;
+    constexpr uint32_t off = s == 0 ? 1u << W : 1u << (W - 1);
+    if constexpr (s == 0) {
+        constexpr int sh = 62 - W - 32;
+        w = ((uint32_t)(u0 >> 32) >> sh) | (((uint32_t)(u1 >> 32) >> sh) << 16);
+    } else if constexpr (W == 8) {
+        constexpr int b = 7 - s;  // byte of the shifted value
+        constexpr uint32_t c = b % 4;
+        const uint32_t x0 = (uint32_t)(b >= 4 ? u0 >> 32 : u0), x1 = (uint32_t)(b >= 4 ? u1 >> 32 : u1);
+        w = __byte_perm(x0, x1, c | (c << 4) | ((4 + c) << 8) | ((4 + c) << 12)) & 0x00FF00FFu;
+    } else {
+        constexpr int sh = 62 - W * (s + 1);
+        w = __byte_perm((uint32_t)(u0 >> sh), (uint32_t)(u1 >> sh), 0x5410) & 0x007F007Fu;
+    }
+    w |= 0x64006400u;
+    const uint32_t k = 0x64006400u + off * 0x00010001u;
+    const __half2 d = __hsub2(*reinterpret_cast<const __half2 *>(&w), *reinterpret_cast<const __half2 *>(&k));
+    return *reinterpret_cast<const uint32_t *>(&d);
 }
 // f(integral_constant<int, s>) for s = 0 .. N-1, unrolled at compile time.
 template <int N, int s = 0, typename F>
@@ -629,16 +610,15 @@ __device__ __forceinline__ void oz_static_for(F &&f) {
     }
 }
 
-// Three bf16 pieces of a float: x = hi + mid + lo (to ~2^-24 relative).
-__device__ __forceinline__ void bf3_pieces(float x, uint32_t (&p)[8]) {
-    __nv_bfloat16 h = __float2bfloat16_rn(x);
-    float r = x - __bfloat162float(h);
-    __nv_bfloat16 m = __float2bfloat16_rn(r);
-    r = r - __bfloat162float(m);
-    __nv_bfloat16 l = __float2bfloat16_rn(r);
-    p[0] = __bfloat16_as_ushort(h);
-    p[1] = __bfloat16_as_ushort(m);
-    p[2] = __bfloat16_as_ushort(l);
+// Three bf16 pieces of two floats: x = hi + mid + lo (to ~2^-24 relative).
+__device__ __forceinline__ void bf3_pairs(float x0, float x1, uint32_t (&p)[3]) {
+#pragma unroll
+    for (int s = 0; s < 3; ++s) {
+        const __nv_bfloat162 h = __floats2bfloat162_rn(x0, x1);
+        p[s] = *reinterpret_cast<const uint32_t *>(&h);
+        x0 -= __uint_as_float(p[s] << 16);
+        x1 -= __uint_as_float(p[s] & 0xFFFF0000u);
+    }
 }
 
 template <typename T>
@@ -668,165 +648,190 @@ struct OzIn<float2> {
     __device__ static float im(float2 v) { return v.y; }
 };
 
-// BF3 = true: float inputs split into bf16 pieces; otherwise Ozaki digits.
-template <typename T, int KT>
-struct SliceSmem {
-    T tile[32][KT + 1];
-    int64_t roff[32], koff[KT];
-    int rexp[32];
+// A slicer tile: 32 rows by 128 embedded columns (128 k, or 64 complex ones),
+// staged in shared memory in 16-byte chunks. A row's chunks are permuted so
+// that a thread's own (8 embedded columns, CPT consecutive chunks) and a
+// column of rows both spread over the banks.
+// Four blocks per SM (64 registers, a few spilled for complex operands): 3.07 ms
+// for the pre-pass of a 4.8 GB Float64 operand, 3.22 with three (80 registers)
+constexpr int OZ_SLICE_OCC = 4;
+__host__ __device__ constexpr int oz_slice_kt(bool cx) { return cx ? 64 : 128; }  // k per tile
+template <typename T, bool CX>
+struct SliceTile {
+    static constexpr int KT = oz_slice_kt(CX);
+    static constexpr int PITCH = KT * (int)sizeof(T);           // bytes per row
+    static constexpr int EPT = CX ? 4 : 8;                      // elements per thread and row
+    static constexpr int CPT = EPT * (int)sizeof(T) / 16;       // their 16-byte chunks
+    static constexpr int VE = 16 / (int)sizeof(T);              // elements per chunk
+    __device__ static int at(int r, int c) { return r * PITCH + ((c & ~7) | ((c ^ ((c >> 3) & (CPT - 1)) ^ r) & 7)) * 16; }
 };
-// k per slicer tile: eight loads per thread before the barrier
-constexpr int OZ_SLICE_KT = 64;
-template <typename T, int MODE>
-using SliceSmemOf = SliceSmem<T, OZ_SLICE_KT>;
-
-// BF16x3: three bf16 pieces per float, one thread per (row, k word).
-template <typename T, int MODE>
-__device__ __forceinline__ void oz_write_pieces(const SliceSmemOf<T, MODE> &sm, const OpGeom &g, uint32_t *outl,
-                                                int64_t plane, int64_t kw, int64_t r0, int64_t k0) {
-    const int tx = threadIdx.x % 32, ty = threadIdx.x / 32;
-    for (int j = 0; j < 4; ++j) {
-        const int r = ty + 8 * j;
-        const int64_t row = r0 + r;
-        if (row >= g.R) continue;
-        if constexpr (MODE == MODE_REAL) {
-            const int64_t word = k0 / 2 + tx;
-            if (word >= kw) continue;
-            uint32_t *o = outl + row * kw + word;
-            uint32_t p0[8], p1[8];
-            bf3_pieces((float)OzIn<T>::re(sm.tile[r][2 * tx]), p0);
-            bf3_pieces((float)OzIn<T>::re(sm.tile[r][2 * tx + 1]), p1);
-#pragma unroll
-            for (int s = 0; s < 3; ++s) o[s * plane] = pack2(p0[s], p1[s]);
-        } else {
-#pragma unroll
-            for (int h = 0; h < 2; ++h) {
-                const int kk = tx + 32 * h;
-                const int64_t word = k0 + kk;
-                if (word >= kw) continue;
-                // MODE_CA: row r; MODE_CB: rows 2r (re, -im) and 2r + 1 (im, re)
-                uint32_t *o = outl + (MODE == MODE_CB ? 2 * row : row) * kw + word;
-                const T v = sm.tile[r][kk];
-                uint32_t pr[8], pi[8], pn[8];
-                bf3_pieces((float)OzIn<T>::re(v), pr);
-                bf3_pieces((float)OzIn<T>::im(v), pi);
-                bf3_pieces(-(float)OzIn<T>::im(v), pn);
-#pragma unroll
-                for (int s = 0; s < 3; ++s) {
-                    if (MODE == MODE_CA) {
-                        o[s * plane] = pack2(pr[s], pi[s]);
-                    } else {
-                        o[s * plane] = pack2(pr[s], pn[s]);
-                        o[s * plane + kw] = pack2(pi[s], pr[s]);
-                    }
-                }
-            }
-        }
-    }
+template <typename T, bool CX>
+struct SliceSmem {
+    alignas(16) unsigned char tile[32 * SliceTile<T, CX>::PITCH];
+    int64_t roff[32], koff[SliceTile<T, CX>::KT];
+    int rowc[32];
+};
+static int64_t oz_slice_tiles(bool cx, int64_t R, int64_t K) {
+    return ((R + 31) / 32) * ((K + oz_slice_kt(cx) - 1) / oz_slice_kt(cx));
+}
+// 16-byte vectors of an operand along k: k's fastest mode is contiguous, and
+// every vector of it starts on a 16-byte boundary when the base does.
+static int oz_kvec(const ModeGroup &gr, const ModeGroup &gk, const ModeGroup &gl, int t, int dtype) {
+    const int64_t ve = 16 / elem_bytes(dtype);
+    if (gk.n == 0 || gk.str[t][0] != 1 || gk.ext[0] % ve) return 0;
+    for (int i = 1; i < gk.n; ++i)
+        if (gk.str[t][i] % ve) return 0;
+    for (int i = 0; i < gr.n; ++i)
+        if (gr.str[t][i] % ve) return 0;
+    for (int i = 0; i < gl.n; ++i)
+        if (gl.str[t][i] % ve) return 0;
+    return 1;
 }
 
-// Ozaki digits with the slice count fixed at compile time: every digit plane
-// is written as soon as it is known, from two biased fixed-point values per
-// thread.
-template <int S, typename T, int MODE>
-__device__ __forceinline__ void oz_write_digits(const SliceSmemOf<T, MODE> &sm, const OpGeom &g, uint32_t *outl,
-                                                int64_t plane, int64_t kw, int64_t r0, int64_t k0) {
-    constexpr int W = oz_digit_bits(S);
-    constexpr int64_t bias = oz_digit_bias(S, W);
-    const int tx = threadIdx.x % 32, ty = threadIdx.x / 32;
-    for (int j = 0; j < 4; ++j) {
-        const int r = ty + 8 * j;
-        const int64_t row = r0 + r;
-        if (row >= g.R) continue;
-        int e = sm.rexp[r];
-        const bool bad = e == 0x7FFFFFFF;
-        if (bad) e = 0;
-        if constexpr (MODE == MODE_REAL) {
-            const int64_t word = k0 / 2 + tx;
-            if (word >= kw) continue;
-            uint32_t *o = outl + row * kw + word;
-            const int64_t q0 = oz_fixed(bad ? 0.0 : (double)OzIn<T>::re(sm.tile[r][2 * tx]), e) + bias;
-            const int64_t q1 = oz_fixed(bad ? 0.0 : (double)OzIn<T>::re(sm.tile[r][2 * tx + 1]), e) + bias;
-            oz_static_for<S>([&](auto sc) {
-                constexpr int s = decltype(sc)::value;
-                o[s * plane] = pack_bf16x2(oz_digit_f<W, s>(q0), oz_digit_f<W, s>(q1));
-            });
-        } else {
-#pragma unroll 1
-            for (int h = 0; h < 2; ++h) {
-                const int kk = tx + 32 * h;
-                const int64_t word = k0 + kk;
-                if (word >= kw) continue;
-                uint32_t *o = outl + (MODE == MODE_CB ? 2 * row : row) * kw + word;
-                const T v = sm.tile[r][kk];  // one shared-memory read of the whole element
-                const int64_t qr = oz_fixed(bad ? 0.0 : (double)OzIn<T>::re(v), e) + bias;
-                const int64_t qi = oz_fixed(bad ? 0.0 : (double)OzIn<T>::im(v), e) + bias;
-                oz_static_for<S>([&](auto sc) {
-                    constexpr int s = decltype(sc)::value;
-                    const float dr = oz_digit_f<W, s>(qr), di = oz_digit_f<W, s>(qi);
-                    if constexpr (MODE == MODE_CA) {
-                        o[s * plane] = pack_bf16x2(dr, di);
-                    } else {
-                        o[s * plane] = pack_bf16x2(dr, oz_digit_f<W, s, true>(qi));
-                        o[s * plane + kw] = pack_bf16x2(di, dr);
-                    }
-                });
-            }
-        }
+// BYTES from global to shared memory; zeros when !in
+template <int BYTES>
+__device__ __forceinline__ void cp_async_zfill(uint32_t dst, const void *src, bool in) {
+    asm volatile("cp.async.ca.shared.global [%0], [%1], %2, %3;" ::"r"(dst), "l"(src), "n"(BYTES), "r"(in ? BYTES : 0)
+                 : "memory");
+}
+
+// The thread's 8 embedded columns of one row (four pairs) as S planes of 16
+// bytes: digits or pieces of consecutive k (MODE_REAL), of (re, im)
+// (MODE_CA), or for the two rows (re, -im) and (im, re) (MODE_CB).
+template <int MODE>
+__device__ __forceinline__ void oz_store_plane(uint32_t *o, int64_t kw, const uint32_t (&w)[4]) {
+    if constexpr (MODE == MODE_CB) {
+        *reinterpret_cast<uint4 *>(o) =
+            make_uint4(w[0] ^ 0x80000000u, w[1] ^ 0x80000000u, w[2] ^ 0x80000000u, w[3] ^ 0x80000000u);
+        *reinterpret_cast<uint4 *>(o + kw) =
+            make_uint4(__byte_perm(w[0], 0, 0x1032), __byte_perm(w[1], 0, 0x1032), __byte_perm(w[2], 0, 0x1032),
+                       __byte_perm(w[3], 0, 0x1032));
+    } else {
+        *reinterpret_cast<uint4 *>(o) = make_uint4(w[0], w[1], w[2], w[3]);
     }
+}
+template <int S, typename X, int MODE>
+__device__ __forceinline__ void oz_write_digits(const X (&x)[8], int rowc, uint32_t *o, int64_t plane, int64_t kw) {
+    constexpr int W = oz_digit_bits(S);
+    constexpr uint64_t bias = oz_digit_bias(S, W);
+    uint64_t u[8];
+#pragma unroll
+    for (int i = 0; i < 8; ++i) u[i] = oz_biased((double)x[i], rowc, bias);
+    oz_static_for<S>([&](auto sc) {
+        constexpr int s = decltype(sc)::value;
+        uint32_t w[4];
+#pragma unroll
+        for (int i = 0; i < 4; ++i) w[i] = oz_digit_pair<W, s>(u[2 * i], u[2 * i + 1]);
+        oz_store_plane<MODE>(o, kw, w);
+        o += plane;
+        if constexpr (s == 0 && W == 8) {
+#pragma unroll
+            for (int i = 0; i < 8; ++i) u[i] <<= 2;
+        }
+    });
 }
 
 // One 32-row tile of an operand: staged through shared memory (coalesced
-// reads whichever mode is contiguous), then written as digit (or piece)
-// planes [L][S][rows_e][kw] with K contiguous.
+// reads whichever mode is contiguous, asynchronous, 16 bytes at a time where
+// k runs contiguously on 16-byte boundaries), then written as digit (or
+// piece) planes [L][S][rows_e][kw] with K contiguous, 16 bytes per thread and
+// plane. BF3: float inputs split into bf16 pieces, otherwise Ozaki digits.
+// HBM bounds it now: the pre-pass of a 4.8 GB Float64 operand takes 3.07 ms
+// (scan and slices; 2.5 at the copy rate) and took 6.65 with a shift, a mask
+// and a float add per digit and 4-byte stores (134 instructions per element).
 template <typename T, int MODE, bool BF3>
 __device__ __forceinline__ void oz_slice_tile(const T *__restrict__ X, const OpGeom &g,
                                               const int32_t *__restrict__ exps, int S,
                                               uint32_t *__restrict__ out, int64_t rows_e, int64_t kw, int64_t blk,
-                                              int64_t l, SliceSmemOf<T, MODE> &sm) {
-    constexpr int KT = OZ_SLICE_KT;
-    int64_t tiles_k = (g.K + KT - 1) / KT;
-    int64_t tr = blk / tiles_k, tk = blk - tr * tiles_k;
-    int64_t r0 = tr * 32, k0 = tk * KT;
-    int tid = threadIdx.x;
+                                              int64_t l, SliceSmem<T, MODE != MODE_REAL> &sm) {
+    using ST = SliceTile<T, MODE != MODE_REAL>;
+    constexpr int KT = ST::KT, ES = (int)sizeof(T);
+    const int64_t tiles_k = (g.K + KT - 1) / KT;
+    const int64_t tr = blk / tiles_k, tk = blk - tr * tiles_k;
+    const int64_t r0 = tr * 32, k0 = tk * KT;
+    const int tid = threadIdx.x;
     if (tid < 32) {
         sm.roff[tid] = (r0 + tid < g.R) ? group_offset(g.gr, g.t, r0 + tid) : 0;
         if (!BF3) {
-            int be = (r0 + tid < g.R) ? exps[l * g.R + r0 + tid] : 0;
-            sm.rexp[tid] = be == 0x7FF ? 0x7FFFFFFF : (be == 0 ? -1022 : be - 1022);
+            const int be = (r0 + tid < g.R) ? exps[l * g.R + r0 + tid] : 0;
+            sm.rowc[tid] = be == 0x7FF ? 10000 : be + 1;
         }
     }
-    if (tid < KT) sm.koff[tid] = (k0 + tid < g.K) ? group_offset(g.gk, g.t, k0 + tid) : 0;
+    if (tid >= 128 && tid - 128 < KT) sm.koff[tid - 128] = (k0 + tid - 128 < g.K) ? group_offset(g.gk, g.t, k0 + tid - 128) : 0;
     const T *Xl = g.ptrs ? (const T *)g.ptrs[l] : X + group_offset(g.gl, g.t, l);
     __syncthreads();
-    for (int idx = tid; idx < 32 * KT; idx += 256) {
-        int r, kk;
-        if (g.rows_fast) {
-            r = idx % 32;
-            kk = idx / 32;
-        } else {
-            kk = idx % KT;
-            r = idx / KT;
-        }
-        T v;
-        memset(&v, 0, sizeof(T));
-        if (r0 + r < g.R && k0 + kk < g.K) v = __ldg(Xl + sm.roff[r] + sm.koff[kk]);
-        sm.tile[r][kk] = v;
+    const int nr = (int)min((int64_t)32, g.R - r0), nk = (int)min((int64_t)KT, g.K - k0);
+    const uint32_t tile = smem_u32(sm.tile);
+    if (g.rows_fast) {
+        const int r = tid % 32;
+        const T *x = Xl + sm.roff[r];
+#pragma unroll 8
+        for (int k = tid / 32; k < KT; k += 8)
+            cp_async_zfill<ES>(tile + ST::at(r, k * ES / 16) + (k * ES) % 16, x + sm.koff[k], r < nr && k < nk);
+    } else if (ES < 16 && g.kvec && ((uintptr_t)Xl & 15) == 0) {
+        constexpr int NC = KT / ST::VE;
+        const int c = tid % NC;
+        const T *x = Xl + sm.koff[c * ST::VE];
+#pragma unroll
+        for (int r = tid / NC; r < 32; r += 256 / NC)
+            cp_async_zfill<16>(tile + ST::at(r, c), x + sm.roff[r], r < nr && c * ST::VE < nk);
+    } else {
+        const int k = tid % KT;
+        const T *x = Xl + sm.koff[k];
+#pragma unroll 8
+        for (int r = tid / KT; r < 32; r += 256 / KT)
+            cp_async_zfill<ES>(tile + ST::at(r, k * ES / 16) + (k * ES) % 16, x + sm.roff[r], r < nr && k < nk);
     }
+    asm volatile("cp.async.wait_all;" ::: "memory");
     __syncthreads();
     const int64_t plane = rows_e * kw;
     uint32_t *outl = out + l * (int64_t)S * plane;
-    if constexpr (BF3) {
-        oz_write_pieces<T, MODE>(sm, g, outl, plane, kw, r0, k0);
-    } else {
-        switch (S) {
-        case 3: oz_write_digits<3, T, MODE>(sm, g, outl, plane, kw, r0, k0); break;
-        case 4: oz_write_digits<4, T, MODE>(sm, g, outl, plane, kw, r0, k0); break;
-        case 5: oz_write_digits<5, T, MODE>(sm, g, outl, plane, kw, r0, k0); break;
-        case 6: oz_write_digits<6, T, MODE>(sm, g, outl, plane, kw, r0, k0); break;
-        case 7: oz_write_digits<7, T, MODE>(sm, g, outl, plane, kw, r0, k0); break;
-        case 8: oz_write_digits<8, T, MODE>(sm, g, outl, plane, kw, r0, k0); break;
-        default: break;  // plans hold 3..8
+    const int col = tid % 16;
+    const int64_t word = (tk * 128 + 8 * col) / 2;
+    if (word >= kw) return;  // kw is a multiple of 4 words: 16 bytes fit or none
+#pragma unroll 1
+    for (int r = tid / 16; r < nr; r += 16) {
+        // 8 embedded columns: components in order
+        using F = decltype(OzIn<T>::re(T()));
+        F x[8];
+        uint4 raw[ST::CPT];
+#pragma unroll
+        for (int j = 0; j < ST::CPT; ++j)
+            raw[j] = *reinterpret_cast<const uint4 *>(sm.tile + ST::at(r, col * ST::CPT + j));
+        if constexpr (MODE == MODE_REAL || OzIn<T>::cx) {
+            static_assert(sizeof(x) == sizeof(raw), "a thread's chunks");
+            memcpy(x, raw, sizeof(x));
+        } else {  // a real operand of a complex contraction: zero imaginary parts
+            F re[4];
+            static_assert(sizeof(re) == sizeof(raw), "a thread's chunks");
+            memcpy(re, raw, sizeof(re));
+#pragma unroll
+            for (int i = 0; i < 4; ++i) {
+                x[2 * i] = re[i];
+                x[2 * i + 1] = F(0);
+            }
+        }
+        uint32_t *o = outl + (MODE == MODE_CB ? 2 : 1) * (r0 + r) * kw + word;
+        if constexpr (BF3) {
+            uint32_t p[4][3];
+#pragma unroll
+            for (int i = 0; i < 4; ++i) bf3_pairs((float)x[2 * i], (float)x[2 * i + 1], p[i]);
+#pragma unroll
+            for (int s = 0; s < 3; ++s) {
+                const uint32_t w[4] = {p[0][s], p[1][s], p[2][s], p[3][s]};
+                oz_store_plane<MODE>(o + s * plane, kw, w);
+            }
+        } else {
+            const int rowc = sm.rowc[r];
+            switch (S) {
+            case 3: oz_write_digits<3, F, MODE>(x, rowc, o, plane, kw); break;
+            case 4: oz_write_digits<4, F, MODE>(x, rowc, o, plane, kw); break;
+            case 5: oz_write_digits<5, F, MODE>(x, rowc, o, plane, kw); break;
+            case 6: oz_write_digits<6, F, MODE>(x, rowc, o, plane, kw); break;
+            case 7: oz_write_digits<7, F, MODE>(x, rowc, o, plane, kw); break;
+            case 8: oz_write_digits<8, F, MODE>(x, rowc, o, plane, kw); break;
+            default: break;  // plans hold 3..8
+            }
         }
     }
 }
@@ -842,14 +847,14 @@ __device__ __forceinline__ void oz_clear_counters(int32_t *cnt, int n) {
 // Slices of both operands (see PrePair). With an adaptive choice the slice
 // count is read from it, and the launch does nothing when it is 0 (plain).
 template <typename T, bool CX, bool BF3>
-__global__ void __launch_bounds__(256, 4) k_oz_slice(const __grid_constant__ PrePair a, int only) {
+__global__ void __launch_bounds__(256, OZ_SLICE_OCC) k_oz_slice(const __grid_constant__ PrePair a, int only) {
     int S = a.S;
     if (a.sel) {
         S = *a.sel;
         if (S == 0) return;
     }
     if (blockIdx.x == 0 && blockIdx.y == 0) oz_clear_counters(a.cnt, a.ncnt);
-    __shared__ SliceSmemOf<T, MODE_REAL> sm;
+    __shared__ SliceSmem<T, CX> sm;
     int64_t blk;
     if (pre_operand(a, only, blk) == 0) {
         const PreOperand &p = a.op[0];
@@ -1151,11 +1156,16 @@ int ozaki_prepass(const ContractionPlan &p, const void *A, const void *B, void *
         q.part = o ? area.partb : area.parta;
         q.out = (uint32_t *)(w + (o ? p.ws_b : p.ws_a));
         q.rows_e = o ? p.n_e : p.m_e;
-        static_assert(OZ_SCAN_KT == OZ_SLICE_KT, "the scan and the slicer walk the same tiles");
-        q.tiles = ((q.g.R + 31) / 32) * ((p.K + OZ_SLICE_KT - 1) / OZ_SLICE_KT);
+        q.g.scan_lk = oz_scan_lk(p.K);
+        q.g.kvec = oz_kvec(q.g.gr, p.gk, p.gl, o, o ? p.b.dtype : p.a.dtype);
     }
-    if (pre.op[0].tiles + pre.op[1].tiles > INT32_MAX)
-        return fail(MGB_ERR_UNSUPPORTED, "operand too large for the slicer grid");
+    auto set_tiles = [&](bool scan) -> int {
+        for (PreOperand &q : pre.op)
+            q.tiles = scan ? oz_scan_tiles(q.g.R, p.K, q.g.scan_lk) : oz_slice_tiles(cx, q.g.R, p.K);
+        if (pre.op[0].tiles + pre.op[1].tiles > INT32_MAX)
+            return fail(MGB_ERR_UNSUPPORTED, "operand too large for the pre-pass grid");
+        return MGB_OK;
+    };
     pre.emax = area.st ? area.st->emax : nullptr;
     pre.kw = p.kpad / 2;
     pre.sel = area.st ? &area.st->sel : nullptr;
@@ -1172,6 +1182,7 @@ int ozaki_prepass(const ContractionPlan &p, const void *A, const void *B, void *
             end = p.K > 1 ? (uint64_t)((uint8_t *)area.qa - w) + 2 * (uint64_t)p.L * sizeof(double)
                           : (uint64_t)((uint8_t *)(area.pb + p.L) - w);
         MGB_CUDA_CHECK(cudaMemsetAsync(w + p.ws_scale_a, 0, end - p.ws_scale_a, s));
+        if (int st = set_tiles(true)) return st;
         int st = by_operand(p, [&](auto tag, int o) -> int {
             k_oz_scale<TypeOf<decltype(tag)>><<<grid(o), 256, 0, s>>>(pre, o);
             MGB_CUDA_CHECK(cudaGetLastError());
@@ -1203,6 +1214,7 @@ int ozaki_prepass(const ContractionPlan &p, const void *A, const void *B, void *
             MGB_CUDA_CHECK(cudaGetLastError());
         }
     }
+    if (int st = set_tiles(false)) return st;
     return by_operand(p, [&](auto tag, int o) -> int {
         using T = TypeOf<decltype(tag)>;
         if (exact) {
@@ -1499,9 +1511,9 @@ __global__ void __launch_bounds__(256, 4) k_oz_scale_multi(const PreJob *__restr
 // Slicing over a table of operand jobs of one element type, embedding and
 // form, as the single-plan slicer does it.
 template <typename T, int MODE, bool BF3>
-__global__ void __launch_bounds__(256, 4) k_oz_slice_multi(const PreJob *__restrict__ jobs,
+__global__ void __launch_bounds__(256, OZ_SLICE_OCC) k_oz_slice_multi(const PreJob *__restrict__ jobs,
                                                         const int64_t *__restrict__ start, int njobs) {
-    __shared__ SliceSmemOf<T, MODE> sm;
+    __shared__ SliceSmem<T, MODE != MODE_REAL> sm;
     const int j = multi_job(start, njobs, blockIdx.x);
     const PreJob &J = jobs[j];
     int S = J.S;
@@ -1591,6 +1603,8 @@ static void fill_prejob(PreJob &J, const ContractionPlan &p, int t, const void *
     J.g.R = t == 0 ? p.M : p.N;
     J.g.K = p.K;
     J.g.rows_fast = unit_row_fast(J.g.gr, p.gk, t);
+    J.g.scan_lk = oz_scan_lk(p.K);
+    J.g.kvec = oz_kvec(J.g.gr, p.gk, p.gl, t, t == 0 ? p.a.dtype : p.b.dtype);
     J.X = X;
     J.dtype = t == 0 ? p.a.dtype : p.b.dtype;
     J.mode = cx ? (t == 0 ? MODE_CA : MODE_CB) : MODE_REAL;
@@ -1628,9 +1642,9 @@ static void fill_prejob(PreJob &J, const ContractionPlan &p, int t, const void *
         }
     }
     J.tiles[PRE_ZERO] = zw ? std::min<int64_t>((zw + 1023) / 1024, 64) : 0;
-    J.tiles[PRE_SCALE] = exact ? ((R + 31) / 32) * ((K + OZ_SCAN_KT - 1) / OZ_SCAN_KT) * L : 0;
+    J.tiles[PRE_SCALE] = exact ? oz_scan_tiles(R, K, J.g.scan_lk) * L : 0;
     J.tiles[PRE_STAT] = (exact && p.adaptive) ? oz_stat_blocks(R, K) * L : 0;
-    J.tiles[PRE_SLICE] = ((R + 31) / 32) * ((K + OZ_SLICE_KT - 1) / OZ_SLICE_KT) * L;
+    J.tiles[PRE_SLICE] = oz_slice_tiles(cx, R, K) * L;
 }
 
 // The chooser's job for an adaptive plan whose statistics lie in `ws`.
