@@ -109,7 +109,9 @@ int mgb_contract(mgb_plan plan, const void *A, const void *B, void *C,
  * Float64 / ComplexF64 sums are fixed-point integers rounded once: exact
  * while the terms lie within 10 binades of the largest one (otherwise within
  * 2^-62 of the largest term per term), independent of the summation order,
- * Inf / NaN as in an FP64 sum. Float32 / ComplexF32 add in FP32.           */
+ * Inf / NaN as in an FP64 sum. Float32 / ComplexF32 add in FP32. The
+ * workspace (mgb_plan_workspace_size bytes, 16-byte aligned) may be missing
+ * or smaller: few outputs of many terms are then summed more slowly.       */
 int mgb_unary_plan(mgb_plan *plan, const mgb_tensor_desc *x,
                    const mgb_tensor_desc *y);
 int mgb_unary(mgb_plan plan, const void *X, void *Y, void *workspace,

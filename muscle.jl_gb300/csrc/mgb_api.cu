@@ -311,7 +311,7 @@ int mgb_plan_destroy(mgb_plan plan) {
 
 int mgb_plan_workspace_size(mgb_plan plan, uint64_t *bytes) {
     if (!plan || !bytes) return fail(MGB_ERR_ARGUMENT, "null argument");
-    *bytes = plan->kind == PlanKind::Contraction ? plan->cp.ws_bytes : 0;
+    *bytes = plan->kind == PlanKind::Contraction ? plan->cp.ws_bytes : unary_workspace(plan->up);
     return MGB_OK;
 }
 
@@ -324,6 +324,7 @@ int mgb_plan_info_get(mgb_plan plan, mgb_plan_info *info) {
         info->n = info->batch = 1;
         info->form = MGB_FORM_PLAIN;
         info->compute_dtype = plan->up.x.dtype;
+        info->workspace_bytes = unary_workspace(plan->up);
         info->flops = (double)plan->up.O * (double)plan->up.R * (is_complex(plan->up.x.dtype) ? 2 : 1);
         return MGB_OK;
     }
@@ -512,13 +513,11 @@ int mgb_unary_plan(mgb_plan *plan, const mgb_tensor_desc *x, const mgb_tensor_de
 
 int mgb_unary(mgb_plan plan, const void *X, void *Y, void *workspace, uint64_t workspace_bytes,
               void *stream) {
-    (void)workspace;
-    (void)workspace_bytes;
     if (!plan || plan->kind != PlanKind::Unary) return fail(MGB_ERR_ARGUMENT, "not a unary plan");
     const UnaryPlan &up = plan->up;
     if (up.O == 0) return MGB_OK;
     if (!X || !Y) return fail(MGB_ERR_ARGUMENT, "null operand pointer");
-    return launch_unary(up, X, Y, (cudaStream_t)stream);
+    return launch_unary(up, X, Y, workspace, workspace_bytes, (cudaStream_t)stream);
 }
 
 int mgb_selftest_wait_timeout(void *stream) { return selftest_wait_timeout((cudaStream_t)stream); }

@@ -109,6 +109,105 @@ MGB_HD void fx_merge(FxSum &a, FxSum b) {
     a.flags |= b.flags;
 }
 
+// A running sum as the reduction kernels keep it: A = lo + hi * 2^32 + neg.
+// Each value's aligned magnitude, two 32-bit words, is complemented when it is
+// negative (~c = -c - 1; `neg` counts the missing ones) and its words go to two
+// 64-bit sums, one multiply-add each on the FMA pipe: the 128-bit add with its
+// carries and sign extension costs twice as many instructions on the integer
+// ALU, the pipe that bounds these sums. Values are aligned to the largest
+// exponent of a group first, so that the rare work (a new largest exponent,
+// Inf, NaN) is one test per group. Words stay below 2^32, so 2^31 values fit.
+// Values within kFxFrac binades of the largest are exact as in fx_push;
+// smaller ones are truncated towards zero.
+struct FxAcc {
+    uint64_t lo;
+    int64_t hi;
+    int32_t neg;
+    int32_t e;
+    uint32_t flags;
+    uint32_t one;  // 1, opaque to the compiler (it would turn the multiply-adds into adds)
+};
+
+MGB_HD FxAcc fx_acc_zero() {
+    uint32_t one;
+#if defined(__CUDA_ARCH__)
+    asm volatile("mov.u32 %0, 1;" : "=r"(one));
+#else
+    one = 1;
+#endif
+    return FxAcc{0ull, 0ll, 0, 1, 0u, one};
+}
+MGB_HD FxSum fx_acc_sum(const FxAcc &a) {
+    FxSum r{0ull, 0ll, a.e, a.flags};
+    fx_add128(r, a.lo, 0ull);
+    fx_add128(r, (uint64_t)a.hi << 32, (uint64_t)(a.hi >> 32));
+    fx_add128(r, (uint64_t)(int64_t)a.neg, (uint64_t)((int64_t)a.neg >> 63));
+    return r;
+}
+// Aligns the sum to the larger exponent e.
+MGB_HD void fx_acc_rise(FxAcc &a, int e) {
+    FxSum r = fx_acc_sum(a);
+    fx_shr(r, e - a.e);
+    a.lo = r.lo & 0xFFFFFFFFull;
+    a.hi = (int64_t)((r.lo >> 32) | ((uint64_t)r.hi << 32));
+    a.neg = 0;
+    a.e = e;
+}
+MGB_HD int fx_bexp(uint64_t b) { return (int)((uint32_t)(b >> 52) & 0x7FFu); }
+// Adds a finite value whose biased exponent is at most a.e.
+MGB_HD void fx_acc_add(FxAcc &a, uint64_t b) {
+    const uint32_t bl = (uint32_t)b, bh = (uint32_t)(b >> 32);
+    const int be = (int)((bh >> 20) & 0x7FFu);
+    const uint32_t mh = (bh & 0xFFFFFu) | (be ? 0x100000u : 0u);
+    const uint64_t m = (((uint64_t)mh << 32) | bl) << kFxFrac;  // below 2^63
+    const int d = a.e - (be > 1 ? be : 1);
+    const uint64_t c = m >> (d < 63 ? d : 63);
+    const int32_t s = (int32_t)bh >> 31;
+    const uint32_t cl = (uint32_t)c ^ (uint32_t)s;
+    const int32_t ch = (int32_t)((uint32_t)(c >> 32) ^ (uint32_t)s);
+#if defined(__CUDA_ARCH__)
+    asm("mad.wide.u32 %0, %1, %2, %0;" : "+l"(a.lo) : "r"(cl), "r"(a.one));
+    asm("mad.wide.s32 %0, %1, %2, %0;" : "+l"(a.hi) : "r"(ch), "r"(a.one));
+#else
+    a.lo += cl;
+    a.hi += ch;
+#endif
+    a.neg -= s;
+}
+// Adds N values.
+template <int N>
+MGB_HD void fx_acc_push(FxAcc &a, const double (&x)[N]) {
+    uint64_t b[N];
+    int m = 0;
+#if defined(__CUDA_ARCH__)
+#pragma unroll
+#endif
+    for (int i = 0; i < N; ++i) {
+        b[i] = fx_bits(x[i]);
+        const int be = fx_bexp(b[i]);
+        m = be > m ? be : m;
+    }
+    if (m > a.e) {
+        if (m == 0x7FF) {  // Inf or NaN among them: flags; the others as usual
+            m = 0;
+            for (int i = 0; i < N; ++i) {
+                const int be = fx_bexp(b[i]);
+                if (be == 0x7FF) {
+                    a.flags |= (b[i] & 0xFFFFFFFFFFFFFull) ? kFxNaN : ((b[i] >> 63) ? kFxNegInf : kFxPosInf);
+                    b[i] = 0;
+                } else if (be > m) {
+                    m = be;
+                }
+            }
+        }
+        if (m > a.e) fx_acc_rise(a, m);
+    }
+#if defined(__CUDA_ARCH__)
+#pragma unroll
+#endif
+    for (int i = 0; i < N; ++i) fx_acc_add(a, b[i]);
+}
+
 // A * 2^(e - 1075 - kFxFrac) rounded to float64 (nearest, ties to even),
 // with overflow to infinity and subnormal results; a zero sum gives +0.
 MGB_HD double fx_value(const FxSum &a) {

@@ -181,7 +181,10 @@ int launch_plain_gemm(const ContractionPlan &p, const void *A, const void *B, vo
 // ws_min bytes they are not.
 int launch_ozaki(const ContractionPlan &p, const void *A, const void *B, void *C,
                  void *ws, bool split, cudaStream_t s, cudaEvent_t mid = nullptr);
-int launch_unary(const UnaryPlan &p, const void *X, void *Y, cudaStream_t s);
+// `ws` (nullable): unary_workspace(p) bytes, 16-byte aligned; without it few
+// outputs of many terms are summed by fewer blocks.
+int launch_unary(const UnaryPlan &p, const void *X, void *Y, void *ws, uint64_t ws_bytes, cudaStream_t s);
+uint64_t unary_workspace(const UnaryPlan &p);
 int selftest_wait_timeout(cudaStream_t s);
 // Emulated forms split for groups: the pre-pass of one plan, and one
 // persistent GEMM launch for several plans of one kernel variant (same

@@ -249,7 +249,9 @@ class BackendGB300(Backend):
             raise ArgumentError("unary_einsum!: X and Y must share the element type")
         plan = unary_plan(x.data, x.inds, y.data, y.inds)
         lib = _lib.load()
-        check(lib.mgb_unary(plan.handle, x.data.data_ptr(), y.data.data_ptr(), None, 0,
+        need = plan.workspace_bytes
+        ws, wp = _workspace(need, y.data.device)
+        check(lib.mgb_unary(plan.handle, x.data.data_ptr(), y.data.data_ptr(), wp or None, need,
                             _stream_handle(y.data.device)), lib)
         return y
 
