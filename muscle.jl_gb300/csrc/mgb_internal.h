@@ -96,6 +96,14 @@ ModeGroup fold_group(std::vector<ModeRec> modes, const bool present[3], int prim
 
 enum class PlanKind { Contraction, Unary };
 
+// How the emulated GEMM cuts the tiles of its last wave along K: the first
+// `full` tiles are whole, the others `splits` units of `kbs` k blocks each
+// (splits = 1: none is cut).
+struct OzTiling {
+    int64_t full = 0;
+    int32_t splits = 1, kbs = 0;
+};
+
 // Resolved binary contraction: GEMM view C[l][m][n] = sum_k A[l][m][k] B[l][k][n].
 struct ContractionPlan {
     Desc a, b, c;
@@ -137,11 +145,8 @@ struct ContractionPlan {
     uint64_t ws_bytes = 0, ws_min = 0;
     // workspace layout (byte offsets)
     uint64_t ws_cnt = 0, ws_part = 0;  // counters and sums of split tiles
-    // Tiles of the emulated GEMM's last wave are cut along K: the first
-    // `split_full` tiles are whole, the others `splits` units of `split_kbs`
-    // k blocks each (splits = 1: none is cut).
-    int64_t split_full = 0;
-    int32_t splits = 1, split_kbs = 0;
+    OzTiling tile[2];   // narrow and wide tiles of the emulated GEMM
+    bool wide = false;  // run in wide tiles where the slice count has them (not in a group)
     uint64_t ws_a = 0, ws_b = 0, ws_scale_a = 0, ws_scale_b = 0;
     int64_t kpad = 0;      // padded embedded K of the slice buffers
     int64_t m_e = 0, n_e = 0, k_e = 0;  // embedded GEMM extents

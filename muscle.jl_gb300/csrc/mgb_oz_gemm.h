@@ -1,13 +1,14 @@
 // The tensor-core GEMM of the emulated forms over digit slices (OZAKI) or
 // pieces (BF16X3), shared by its translation units: one contraction of a
 // fixed slice count (mgb_oz_gemm_one.cu), one whose slice count the device
-// chose (mgb_oz_gemm_any.cu), and a table of contractions
-// (mgb_oz_gemm_table.cu).
+// chose (mgb_oz_gemm_any.cu), either in wide tiles (mgb_oz_gemm_wide.cu), and a
+// table of contractions (mgb_oz_gemm_table.cu).
 #pragma once
 
 #include <cuda.h>
 
 #include <atomic>
+#include <type_traits>
 
 #include "mgb_internal.h"
 #include "mgb_ptx.h"
@@ -18,7 +19,6 @@ namespace mgb {
 constexpr int OZ_KC = 256;     // BF16X3: embedded k between readouts
 constexpr int OZ_BM = 128;     // rows of A per CTA (TMEM lanes)
 constexpr int OZ_BK = 32;      // k per stage (64-byte swizzled rows)
-constexpr int OZ_EPI_WARPS = 8;
 // Row tiles per rasterisation band. The resident CTAs drift apart in k over
 // many waves, so L2 keeps a band's A slices only while they are small: on the
 // 8192^3 ComplexF64 case (S = 6) DRAM traffic per launch is 222 GB for bands
@@ -30,21 +30,34 @@ constexpr int OZ_EPI_WARPS = 8;
 // with 3 and 78.0 ms with 2.
 constexpr int OZ_GROUP_M = 3;
 constexpr int64_t OZ_BAND_BYTES = 90ll << 20;  // S = 7 at K_e = 16384: 84 MiB; S = 8: 96 MiB
-// warp 0 TMA, warp 1 MMA issuer (and TMEM owner), warps 2..9 epilogue,
-// warp 10 second MMA issuer
-constexpr int OZ_THREADS = 96 + 32 * OZ_EPI_WARPS;
+// warp 0 TMA, warp 1 MMA issuer (and TMEM owner), warps 2..9 epilogue, warp 10
+// second MMA issuer (narrow tiles)
+constexpr int OZ_EPI_WARPS = 8;
+__host__ __device__ constexpr int oz_threads(bool wide) { return 64 + 32 * OZ_EPI_WARPS + (wide ? 0 : 32); }
 constexpr int OZ_ISSUER2_WARP = 2 + OZ_EPI_WARPS;
 constexpr int OZ_A_TILE = OZ_BM * OZ_BK * 2;  // 8192 bytes per slice
 constexpr int OZ_SMEM_BUDGET = 220 * 1024;
 constexpr int OZ_MAX_STAGES = 6;
+constexpr int OZ_NAN_EXP = 1 << 20;  // exponent of a row or column whose results are NaN
 
 // Columns per digit group (= embedded rows of B per CTA): two banks of S
 // groups must fit the 512 TMEM columns, and one MMA covers at most 256.
 // BF16X3 (S = 3, two float registers per column) takes 64; the exact forms
 // keep 32, where their three 32-bit words per column stay in registers.
-__host__ __device__ constexpr int oz_bn(int S, bool exact) { return (!exact && S <= 3) ? 64 : 32; }
-__host__ __device__ constexpr int oz_b_tile(int S, bool exact) { return oz_bn(S, exact) * OZ_BK * 2; }  // bytes per slice
-__host__ __device__ constexpr int oz_stage_bytes(int S, bool exact) { return S * (OZ_A_TILE + oz_b_tile(S, exact)); }
+// Wide tiles of the exact forms take 64 with one bank (see oz_gemm_body).
+__host__ __device__ constexpr int oz_bn(int S, bool exact, bool wide = false) {
+    return wide || (!exact && S <= 3) ? 64 : 32;
+}
+// Slice counts with wide tiles: 3, and 6, the usual one. With 5 they were 2 to
+// 12 % slower (narrow tiles have a stage more there), with 4 between 3 % faster
+// and 2 % slower; 7 and 8 have no room for three stages.
+__host__ __device__ constexpr bool oz_wide(int S) { return S == 3 || S == 6; }
+__host__ __device__ constexpr int oz_b_tile(int S, bool exact, bool wide = false) {  // bytes per slice
+    return oz_bn(S, exact, wide) * OZ_BK * 2;
+}
+__host__ __device__ constexpr int oz_stage_bytes(int S, bool exact, bool wide = false) {
+    return S * (OZ_A_TILE + oz_b_tile(S, exact, wide));
+}
 // Digit width and exact chunk length (in 32-wide k blocks) per slice count.
 // W = 8 for S <= 6: |s1| <= 256, |si| <= 128, group bound max(d+1,4) 2^14, so a
 // float32 accumulator stays exact over 4 blocks (128 k) for every d <= 7.
@@ -54,16 +67,17 @@ __host__ __device__ constexpr int oz_digit_bits(int S) { return S <= 6 ? 8 : 7; 
 __host__ __device__ constexpr int oz_chunk_blocks(int S) { return oz_digit_bits(S) == 8 ? 4 : 8; }
 // k blocks between readouts
 __host__ __device__ constexpr int oz_chunk(int S, bool exact) { return exact ? oz_chunk_blocks(S) : OZ_KC / OZ_BK; }
-__host__ __device__ constexpr int oz_stages(int S, bool exact) {
-    return (OZ_SMEM_BUDGET / oz_stage_bytes(S, exact)) < OZ_MAX_STAGES ? (OZ_SMEM_BUDGET / oz_stage_bytes(S, exact))
-                                                                       : OZ_MAX_STAGES;
+__host__ __device__ constexpr int oz_stages(int S, bool exact, bool wide = false) {
+    return (OZ_SMEM_BUDGET / oz_stage_bytes(S, exact, wide)) < OZ_MAX_STAGES
+               ? (OZ_SMEM_BUDGET / oz_stage_bytes(S, exact, wide))
+               : OZ_MAX_STAGES;
 }
 // two banks of S groups of oz_bn columns; bank bases at columns 0 and 256
 __host__ __device__ constexpr int oz_tmem_cols(int) { return 512; }
 // More than half of the SM's shared memory for every S, so one CTA (and one
 // TMEM allocation) per SM.
-__host__ __device__ constexpr int oz_smem_bytes(int S, bool exact) {
-    return oz_stages(S, exact) * oz_stage_bytes(S, exact) + 1024 /*align*/ + 256 /*barriers*/;
+__host__ __device__ constexpr int oz_smem_bytes(int S, bool exact, bool wide = false) {
+    return oz_stages(S, exact, wide) * oz_stage_bytes(S, exact, wide) + 1024 /*align*/ + 256 /*barriers*/;
 }
 static_assert(2 * oz_smem_bytes(3, true) > 228 * 1024 && 2 * oz_smem_bytes(8, true) > 228 * 1024 &&
                   2 * oz_smem_bytes(3, false) > 228 * 1024,
@@ -127,15 +141,27 @@ __device__ __forceinline__ void tc_ld(uint32_t taddr, uint32_t (&v)[NC]) {
     asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory");
 }
 
-// 96-bit two's-complement accumulation (carry chain) and conversion.
-__device__ __forceinline__ void add96(uint32_t &w0, uint32_t &w1, uint32_t &w2, uint32_t a0, uint32_t a1,
-                                      uint32_t a2) {
-    asm("add.cc.u32 %0, %0, %3;\n\taddc.cc.u32 %1, %1, %4;\n\taddc.u32 %2, %2, %5;"
-        : "+r"(w0), "+r"(w1), "+r"(w2)
-        : "r"(a0), "r"(a1), "r"(a2));
+// hi:lo += x m over 96 bits
+__device__ __forceinline__ void add96(uint32_t &lo, int64_t &hi, int32_t x, int32_t m) {
+    asm("{\n\t.reg .b64 p;\n\t.reg .b32 a, b, c, l, h;\n\t"
+        "mul.wide.s32 p, %2, %3;\n\t"
+        "mov.b64 {a, b}, p;\n\t"
+        "shr.s32 c, b, 31;\n\t"
+        "mov.b64 {l, h}, %1;\n\t"
+        "add.cc.u32 %0, %0, a;\n\t"
+        "addc.cc.u32 l, l, b;\n\t"
+        "addc.u32 h, h, c;\n\t"
+        "mov.b64 %1, {l, h};\n\t}"
+        : "+r"(lo), "+l"(hi)
+        : "r"(x), "r"(m));
 }
-__device__ __forceinline__ void add64hi(uint32_t &w1, uint32_t &w2, uint32_t a1, uint32_t a2) {
-    asm("add.cc.u32 %0, %0, %2;\n\taddc.u32 %1, %1, %3;" : "+r"(w1), "+r"(w2) : "r"(a1), "r"(a2));
+// f(integral_constant<int, s>) for s = 0 .. N-1, unrolled at compile time.
+template <int N, int s = 0, typename F>
+__device__ __forceinline__ void oz_static_for(F &&f) {
+    if constexpr (s < N) {
+        f(std::integral_constant<int, s>{});
+        oz_static_for<N, s + 1>(f);
+    }
 }
 
 // K-major operand tile, 64-byte swizzle: rows of 64 B, 8-row atoms of 512 B.
@@ -200,6 +226,7 @@ struct OzAnyJob : OzJobShape {
     CUtensorMap tm[6][2];
     int32_t band[6];
     uint32_t cand;
+    int32_t S;  // the count when a.sel is null
 };
 
 // Tile sources of the kernel: one job in the parameter space, or a table of
@@ -368,19 +395,36 @@ __device__ __forceinline__ bool oz_part_last(int32_t *cnt, int tile, int w, int 
 // the exact forms: the widest that two banks leave room for while the
 // epilogue's accumulators (96-bit integers, or float sums and their
 // compensations) stay in registers.
-template <int S, bool EXACT, bool CX, typename Src>
+//
+// WIDE (EXACT, see oz_wide): 128 x 64 tiles. Shared memory bounds the narrow ones:
+// per 16 k a tile's slices are written once and A's are read once, whatever
+// its width, so twice the columns save 26 % of the bytes (112 KB against
+// 2 x 76 at S = 6). Two banks of 64-column groups do not fit TMEM, so there is
+// one, and the readout of a chunk overlaps the MMAs of the next by groups
+// instead of by banks: the epilogue reads, clears and releases the groups from
+// the last to the first, and the issuer starts a chunk with its last A slice,
+// whose products touch the last group only, then the one before it, and so on,
+// each over the chunk's first two k blocks. An MMA covers at most 256 columns,
+// so the first two A slices take two MMAs each. With MMAs this long one issuer
+// keeps the tensor core's queue filled across its polls. 8192^3, S = 6: 18.6 ms
+// in narrow tiles, 16.8 in wide ones (Float64), 75.2 and 67.3 (ComplexF64). A
+// chunk takes 9.4 k cycles, of which the readout 3.3 k; two places for the last
+// two groups, a readout without conversions (eight cycles of their unit per
+// warp) or with more registers, and sixteen epilogue warps were slower.
+template <int S, bool EXACT, bool CX, bool WIDE, typename Src>
 __device__ __forceinline__ void oz_gemm_body(const Src &src) {
     constexpr int W = oz_digit_bits(S);  // digit width (EXACT)
     constexpr int KCB = oz_chunk(S, EXACT);  // k blocks per chunk
-    constexpr int NST = oz_stages(S, EXACT);
-    constexpr int STAGE = oz_stage_bytes(S, EXACT);
-    constexpr int BN = oz_bn(S, EXACT);  // columns per digit group, embedded B rows per CTA
+    constexpr int NST = oz_stages(S, EXACT, WIDE);
+    constexpr int STAGE = oz_stage_bytes(S, EXACT, WIDE);
+    constexpr int BN = oz_bn(S, EXACT, WIDE);  // columns per digit group, embedded B rows per CTA
     constexpr int HALF = BN / 2;     // columns per group read by one epilogue warp
     constexpr int TCOLS = oz_tmem_cols(S);
     constexpr int BANK = TCOLS / 2;  // TMEM column offset of the second bank
     static_assert(NST >= 2, "need at least two pipeline stages");
-    static_assert(BN * S <= BANK && TCOLS <= 512, "two banks must fit in TMEM");
-    static_assert(BN * S <= 256, "one MMA covers at most 256 columns");
+    static_assert(WIDE ? BN * S <= TCOLS : BN * S <= BANK, "the accumulators must fit in TMEM");
+    static_assert(WIDE ? EXACT && oz_wide(S) : BN * S <= 256, "one MMA covers at most 256 columns");
+    static_assert(oz_smem_bytes(S, EXACT, WIDE) <= 227 * 1024, "shared memory of a CTA");
     static_assert(HALF % 16 == 0, "epilogue reads 16 columns at a time");
     // MMA-issuing threads. Each mbarrier poll by an issuing thread stalls it
     // for ~150 cycles while the tensor core's queue holds only ~200 cycles of
@@ -389,7 +433,8 @@ __device__ __forceinline__ void oz_gemm_body(const Src &src) {
     // the other polls. Their MMAs into a bank interleave in an unspecified
     // order, which changes nothing for the exact integer sums of the OZAKI
     // form; BF16X3 sums round, so it keeps one issuer and stays deterministic.
-    constexpr int NI = EXACT ? 2 : 1;
+    constexpr int NI = EXACT && !WIDE ? 2 : 1;
+    constexpr int NF = WIDE ? S : 2;  // accumulator parts released one by one: groups, or banks
 
     extern __shared__ uint8_t smem_raw[];
     uint8_t *smem = (uint8_t *)(((uintptr_t)smem_raw + 1023) & ~(uintptr_t)1023);
@@ -397,8 +442,8 @@ __device__ __forceinline__ void oz_gemm_body(const Src &src) {
     uint64_t *full = bars;               // [2 NST] see full_idx
     uint64_t *empty = bars + 2 * NST;    // [NST]
     uint64_t *acc_full = bars + 3 * NST; // [2] bank filled (one commit per issuer)
-    uint64_t *acc_empty = acc_full + 2;  // [2] bank read and cleared (one arrive per epilogue warp)
-    uint64_t *done = acc_empty + 2;      // [2] per issuer: all its MMAs complete
+    uint64_t *acc_empty = acc_full + 2;  // [NF] part read and cleared (one arrive per epilogue warp)
+    uint64_t *done = acc_empty + NF;     // [2] per issuer: all its MMAs complete
     uint32_t *tmem_slot = (uint32_t *)(done + 2);
     volatile int *abort_flag = (volatile int *)(tmem_slot + 1);
 
@@ -437,9 +482,9 @@ __device__ __forceinline__ void oz_gemm_body(const Src &src) {
         }
         for (int b = 0; b < 2; ++b) {
             mbar_init(smem_u32(acc_full + b), NI);
-            mbar_init(smem_u32(acc_empty + b), OZ_EPI_WARPS);
             mbar_init(smem_u32(done + b), 1);
         }
+        for (int b = 0; b < NF; ++b) mbar_init(smem_u32(acc_empty + b), OZ_EPI_WARPS);
         *abort_flag = 0;
         asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
         asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
@@ -466,8 +511,8 @@ __device__ __forceinline__ void oz_gemm_body(const Src &src) {
     __syncthreads();
     tc_fence_after();
 
-    if (warp == 0) {
-        // ---------------- TMA producer ----------------
+    // ---------------- TMA producer ----------------
+    auto produce = [&]() {
         if (lane == 0) {
             uint32_t g = 0;  // k blocks issued so far, over all tiles of this CTA
             bool ok = true;
@@ -498,8 +543,70 @@ __device__ __forceinline__ void oz_gemm_body(const Src &src) {
             for (uint32_t gg = g > (uint32_t)NST ? g - NST : 0u; gg < g; ++gg)
                 mbar_drain(smem_u32(full + full_idx(gg)), full_par(gg));
         }
-    } else if (warp == 1 || (NI == 2 && warp == OZ_ISSUER2_WARP)) {
-        // ---------------- MMA issuers ----------------
+    };
+    // ---------------- MMA issuer (wide tiles) ----------------
+    auto issue_wide = [&]() {
+        if (lane == 0) {
+            bool ok = true;
+            uint32_t g = 0, C = 0;
+            int hint = 0;
+            // the products of A slice i over 16 k of a stage
+            auto issue = [&](uint32_t stage, int i, int k16) {
+                const uint32_t a_base = smem_u32(smem + stage * STAGE);
+                const uint64_t ad = sw64_desc(a_base) + (uint64_t)((i * OZ_A_TILE + k16 * 32) >> 4);
+                const uint64_t bd = sw64_desc(a_base + S * OZ_A_TILE) + (uint64_t)((k16 * 32) >> 4);
+                // columns of the first MMA: both of a pair at least 128 wide,
+                // below which an MMA waits for A's slice
+                const int n = BN * (S - i), n1 = n > 256 ? 192 : n;
+                tc_mma(tmem + BN * i, ad, bd, oz_idesc(n1, true), 1u);
+                if (n > n1)
+                    tc_mma(tmem + BN * i + n1, ad, bd + (uint64_t)((n1 / BN) * oz_b_tile(S, true, true) >> 4),
+                           oz_idesc(n - n1, true), 1u);
+            };
+            for (int64_t t = blockIdx.x; t < T && ok; t += gridDim.x) {
+                int64_t local;
+                const OzJobShape &J = src.job(t, local, hint);
+                const OzUnit u = oz_unit(J, local, src.band(hint), BN);
+                const int nkb = u.kb1 - u.kb0;
+                for (int c0 = 0; c0 < nkb && ok; c0 += KCB, ++C) {
+                    const int c1 = min(nkb, c0 + KCB), r1 = min(c1, c0 + 2);
+                    for (int kb = c0; kb < r1 && ok; ++kb)
+                        ok = mbar_wait(smem_u32(full + full_idx(g + kb)), full_par(g + kb), abort_flag, status);
+#pragma unroll
+                    for (int i = S - 1; i >= 0; --i) {
+                        // group i of the previous chunk read and cleared
+                        ok = ok && mbar_wait(smem_u32(acc_empty + i), (C & 1u) ^ 1u, abort_flag, status);
+                        if (!ok) break;
+                        tc_fence_after();
+                        for (int kb = c0; kb < r1; ++kb)
+#pragma unroll
+                            for (int k16 = 0; k16 < OZ_BK / 16; ++k16) issue((g + kb) % NST, i, k16);
+                    }
+                    if (!ok) break;
+                    for (int kb = c0; kb < r1; ++kb) tc_commit(smem_u32(empty + (g + kb) % NST));
+                    for (int kb = r1; kb < c1; ++kb) {
+                        if (!mbar_wait(smem_u32(full + full_idx(g + kb)), full_par(g + kb), abort_flag, status)) {
+                            ok = false;
+                            break;
+                        }
+                        tc_fence_after();
+#pragma unroll
+                        for (int k16 = 0; k16 < OZ_BK / 16; ++k16)
+#pragma unroll
+                            for (int i = S - 1; i >= 0; --i) issue((g + kb) % NST, i, k16);
+                        tc_commit(smem_u32(empty + (g + kb) % NST));
+                    }
+                    if (ok) tc_commit(smem_u32(acc_full));
+                }
+                g += (uint32_t)nkb;
+            }
+            // wait for every MMA before TMEM is released
+            tc_commit(smem_u32(done));
+            mbar_drain(smem_u32(done), 0);
+        }
+    };
+    // ---------------- MMA issuers (narrow tiles) ----------------
+    auto issue_narrow = [&]() {
         // Issuer `me` takes the k blocks whose running count g has g % NI == me.
         // Per chunk C (counted over all tiles) it waits until the epilogue has
         // read and cleared the bank's previous chunk (C - 2), issues its k
@@ -555,8 +662,9 @@ __device__ __forceinline__ void oz_gemm_body(const Src &src) {
             tc_commit(smem_u32(done + me));
             mbar_drain(smem_u32(done + me), 0);
         }
-    } else if (warp < 2 + OZ_EPI_WARPS) {
-        // ---------------- epilogue ----------------
+    };
+    // ---------------- epilogue ----------------
+    auto epilogue = [&]() {
         const int q = warp % 4;        // TMEM lane quarter this warp may access
         const int h = (warp - 2) / 4;  // column half (HALF columns) of each group
         const uint32_t tbase = tmem + ((uint32_t)(32 * q) << 16) + HALF * h;
@@ -579,42 +687,47 @@ __device__ __forceinline__ void oz_gemm_body(const Src &src) {
             // Output addressing of the tile, fetched before the first chunk
             // wait so that its loads overlap the MMAs: the thread's row (offset
             // and exponent), and one output column per lane (lane j < NCOL
-            // holds column j of this warp's half, broadcast by shuffles).
+            // holds column j of this warp's half, broadcast by shuffles). A
+            // row or column without finite values has the exponent OZ_NAN_EXP.
             constexpr int NCOL = CX ? HALF / 2 : HALF;
             const bool row_ok = row < args.M;
             int64_t rowoff = 0;
             int erow = 0;
-            bool badrow = false;
             if (row_ok) {
                 rowoff = (args.cptr ? 0 : group_offset(args.gl, 2, l)) + group_offset(args.gm, 2, row);
                 if (EXACT) {
                     const int be = args.expA[(int64_t)l * args.M + row];
-                    badrow = be == 0x7FF;
-                    erow = be == 0 ? -1022 : be - 1022;
+                    erow = be == 0x7FF ? OZ_NAN_EXP : be == 0 ? -1022 : be - 1022;
                 }
             }
             long long lcoff = 0;
-            int lexp = -1;  // the column's exponent (0 without one), -1 beyond the output
+            int lexp = 0;  // the column's exponent and the scale of X's last bit
+            bool lcol = false;
             {
                 const int64_t ne = n0 + HALF * h + (int64_t)lane * (CX ? 2 : 1);
                 if (lane < NCOL && ne < args.Ne) {
                     const int64_t n = CX ? (ne >> 1) : ne;
                     lcoff = group_offset(args.gn, 2, n);
-                    lexp = EXACT ? args.expB[(int64_t)l * args.N + n] : 0;
+                    lcol = true;
+                    if (EXACT) {
+                        const int be = args.expB[(int64_t)l * args.N + n];
+                        lexp = (be == 0x7FF ? OZ_NAN_EXP : be == 0 ? -1022 : be - 1022) - W * (S + 1);
+                    }
                 }
             }
+            const uint32_t cols = __ballot_sync(0xffffffffu, lcol);
             void *const Cl = args.cptr ? args.cptr[l] : args.C;
-            // EXACT: one 96-bit two's-complement integer per output column,
-            // X = sum_d G_d 2^(W (S + 1 - d)), held in w0 (bits 0-31), w1, w2.
-            uint32_t w0[EXACT ? HALF : 1], w1[EXACT ? HALF : 1], w2[EXACT ? HALF : 1];
+            // EXACT: one 96-bit integer X = sum_d G_d 2^(W (S + 1 - d)) per
+            // output column, x0 + x1 2^32
+            uint32_t x0[EXACT ? HALF : 1];
+            int64_t x1[EXACT ? HALF : 1];
             // BF16X3: Kahan-compensated float32 sum over the chunks
             float accf[EXACT ? 1 : HALF], comp[EXACT ? 1 : HALF];
 #pragma unroll
             for (int j = 0; j < HALF; ++j) {
                 if (EXACT) {
-                    w0[j] = 0;
-                    w1[j] = 0;
-                    w2[j] = 0;
+                    x0[j] = 0;
+                    x1[j] = 0;
                 } else {
                     accf[j] = 0.f;
                     comp[j] = 0.f;
@@ -622,44 +735,60 @@ __device__ __forceinline__ void oz_gemm_body(const Src &src) {
             }
 #pragma unroll 1
             for (int c = 0; c < nchunks; ++c, ++C) {
-                const uint32_t bank = C & 1u;
+                const uint32_t bank = WIDE ? 0u : C & 1u;
                 // warp-uniform outcome: the warp-collective loads below need every lane
-                if (!__all_sync(0xffffffffu, mbar_wait(smem_u32(acc_full + bank), (C >> 1) & 1u, abort_flag, status))) {
+                if (!__all_sync(0xffffffffu, mbar_wait(smem_u32(acc_full + bank), (WIDE ? C : C >> 1) & 1u, abort_flag,
+                                                       status))) {
                     ok = false;
                     break;
                 }
                 tc_fence_after();
                 const uint32_t tb = tbase + bank * BANK;
-                if constexpr (EXACT) {
+                // adds 16 columns' partial sums of a group, shifted into place
+                auto add_group = [&](auto gc, auto jc, const uint32_t (&v)[16]) {
+                    constexpr int sh = W * (S - 1 - decltype(gc)::value);  // W (S + 1 - d), d = g + 2
 #pragma unroll
-                    for (int g = 0; g < S; ++g) {
-                        uint32_t v[HALF];
-                        tc_ld<HALF>(tb + BN * g, v);
-#pragma unroll
-                        for (int c2 = 0; c2 < HALF; c2 += 16) tc_st16_zero(tb + BN * g + c2);
-                        if (g == S - 1) {  // every group of the bank read and cleared
+                    for (int j = 0; j < 16; ++j) {
+                        const int32_t x = __float2int_rn(__uint_as_float(v[j]));
+                        const int k = decltype(jc)::value + j;
+                        if constexpr (sh < 32) add96(x0[k], x1[k], x, 1 << sh);
+                        else x1[k] += (int64_t)x << (sh - 32);
+                    }
+                };
+                if constexpr (WIDE) {
+                    oz_static_for<S>([&](auto ic) {
+                        constexpr int g = S - 1 - decltype(ic)::value;  // from the last to the first
+                        const uint32_t at = tb + BN * g;
+                        oz_static_for<HALF / 16>([&](auto hc) {
+                            constexpr int c2 = 16 * decltype(hc)::value;
+                            uint32_t v[16];
+                            tc_ld<16>(at + c2, v);
+                            tc_st16_zero(at + c2);
+                            if constexpr (c2 + 16 == HALF) {  // this warp's share of the group read and cleared
+                                tc_wait_st();
+                                tc_fence_before();
+                                __syncwarp();
+                                if (lane == 0) mbar_arrive(smem_u32(acc_empty + g));
+                            }
+                            add_group(std::integral_constant<int, g>{}, std::integral_constant<int, c2>{}, v);
+                        });
+                    });
+                } else if constexpr (EXACT) {
+                    oz_static_for<S>([&](auto gc) {
+                        constexpr int g = decltype(gc)::value;
+                        uint32_t v[16];
+                        tc_ld<16>(tb + BN * g, v);
+                        tc_st16_zero(tb + BN * g);
+                        if constexpr (g == S - 1) {  // every group of the bank read and cleared
                             tc_wait_st();
                             tc_fence_before();
                             __syncwarp();
                             if (lane == 0) mbar_arrive(smem_u32(acc_empty + bank));
                         }
-                        const int sh = W * (S - 1 - g);  // W (S + 1 - d), d = g + 2
-                        if (sh < 32) {
-#pragma unroll
-                            for (int j = 0; j < HALF; ++j) {
-                                int64_t x = (int64_t)__float2int_rn(__uint_as_float(v[j])) << sh;
-                                add96(w0[j], w1[j], w2[j], (uint32_t)x, (uint32_t)((uint64_t)x >> 32),
-                                      x < 0 ? 0xFFFFFFFFu : 0u);
-                            }
-                        } else {
-#pragma unroll
-                            for (int j = 0; j < HALF; ++j) {
-                                int64_t x = (int64_t)__float2int_rn(__uint_as_float(v[j])) << (sh - 32);
-                                add64hi(w1[j], w2[j], (uint32_t)x, (uint32_t)((uint64_t)x >> 32));
-                            }
-                        }
-                    }
-                } else {
+                        add_group(gc, std::integral_constant<int, 0>{}, v);
+                    });
+                }
+                if constexpr (!EXACT) {
                     // pieces hi*hi, then the products of piece-index sum 1 and 2;
                     // 16 columns at a time, so that the three groups' registers
                     // stay beside the running sums and their compensations
@@ -689,20 +818,35 @@ __device__ __forceinline__ void oz_gemm_body(const Src &src) {
                 }
             }
             if (!ok) break;
+            // column j's X in three words, two's complement
+            struct X96 {
+                uint32_t w0, w1, w2;
+            };
+            auto words = [&](int j) {
+                return X96{x0[j], (uint32_t)x1[j], (uint32_t)((uint64_t)x1[j] >> 32)};
+            };
             if (u.part >= 0) {  // part of a split tile
                 constexpr int NW = EXACT ? 3 * HALF : 2 * HALF;
                 const int w = warp - 2, sp = u.part % args.splits, first = u.part - sp;
                 uint4 *mine = oz_part_at<NW>(args.part, u.part, w);
+                if constexpr (EXACT) {
 #pragma unroll
-                for (int i = 0; i < NW / 4; ++i) {
-                    uint32_t v[4];
-#pragma unroll
-                    for (int e = 0; e < 4; ++e) {
-                        const int k = 4 * i + e;  // a constant: the loops are unrolled
-                        if constexpr (EXACT) v[e] = k < HALF ? w0[k % HALF] : k < 2 * HALF ? w1[k % HALF] : w2[k % HALF];
-                        else v[e] = __float_as_uint(k < HALF ? accf[k % HALF] : comp[k % HALF]);
+                    for (int j0 = 0; j0 < HALF; j0 += 4) {
+                        const X96 a = words(j0), b = words(j0 + 1), c = words(j0 + 2), d = words(j0 + 3);
+                        __stcg(mine + (j0 / 4) * 32, make_uint4(a.w0, b.w0, c.w0, d.w0));
+                        __stcg(mine + ((HALF + j0) / 4) * 32, make_uint4(a.w1, b.w1, c.w1, d.w1));
+                        __stcg(mine + ((2 * HALF + j0) / 4) * 32, make_uint4(a.w2, b.w2, c.w2, d.w2));
                     }
-                    __stcg(mine + i * 32, make_uint4(v[0], v[1], v[2], v[3]));
+                } else {
+#pragma unroll
+                    for (int j0 = 0; j0 < HALF; j0 += 4) {
+                        __stcg(mine + (j0 / 4) * 32,
+                               make_uint4(__float_as_uint(accf[j0]), __float_as_uint(accf[j0 + 1]),
+                                          __float_as_uint(accf[j0 + 2]), __float_as_uint(accf[j0 + 3])));
+                        __stcg(mine + ((HALF + j0) / 4) * 32,
+                               make_uint4(__float_as_uint(comp[j0]), __float_as_uint(comp[j0 + 1]),
+                                          __float_as_uint(comp[j0 + 2]), __float_as_uint(comp[j0 + 3])));
+                    }
                 }
                 if (!oz_part_last(args.cnt, u.part / args.splits, w, args.splits)) continue;
                 if constexpr (EXACT) {  // integers: any order gives the same sum
@@ -714,10 +858,15 @@ __device__ __forceinline__ void oz_gemm_body(const Src &src) {
                         for (int j0 = 0; j0 < HALF; j0 += 4) {
                             const uint4 x = __ldcg(p + (j0 / 4) * 32), y = __ldcg(p + ((HALF + j0) / 4) * 32),
                                         z = __ldcg(p + ((2 * HALF + j0) / 4) * 32);
-                            add96(w0[j0], w1[j0], w2[j0], x.x, y.x, z.x);
-                            add96(w0[j0 + 1], w1[j0 + 1], w2[j0 + 1], x.y, y.y, z.y);
-                            add96(w0[j0 + 2], w1[j0 + 2], w2[j0 + 2], x.z, y.z, z.z);
-                            add96(w0[j0 + 3], w1[j0 + 3], w2[j0 + 3], x.w, y.w, z.w);
+                            const uint32_t xs[4] = {x.x, x.y, x.z, x.w}, ys[4] = {y.x, y.y, y.z, y.w},
+                                           zs[4] = {z.x, z.y, z.z, z.w};
+#pragma unroll
+                            for (int e = 0; e < 4; ++e) {
+                                const int64_t hi = (int64_t)(((uint64_t)zs[e] << 32) | ys[e]);
+                                const uint64_t lo = (uint64_t)x0[j0 + e] + xs[e];
+                                x0[j0 + e] = (uint32_t)lo;
+                                x1[j0 + e] += hi + (int64_t)(lo >> 32);
+                            }
                         }
                     }
                 } else {  // compensated float sums, always in the order of k
@@ -742,62 +891,81 @@ __device__ __forceinline__ void oz_gemm_body(const Src &src) {
                 }
             }
             if constexpr (EXACT) {
-                // Four conversions at a time through the straight-line routine,
-                // so that their integer sequences interleave (one conversion
-                // alone is a chain of dependent instructions); a group with a
-                // subnormal result (rare) goes through the general routine;
-                // then the group's stores.
+                // Four conversions at a time, so that their integer sequences
+                // interleave (one alone is a chain of dependent instructions):
+                // in 64 bits where all of the warp's X fit, as they do unless K
+                // is huge, and through the general routine where an exponent
+                // leaves the plain range. A loop, whose columns move down to
+                // the same registers each time: unrolled, the instructions
+                // alone took longer to fetch than to run. S = 6, a tile's 16
+                // columns per thread: 4800 cycles for 96-bit conversions that
+                // handle every exponent, 2800 so; 4864 tiles of 4 k blocks
+                // 178 -> 151 us, one tile of 4 k blocks (with its launch) 14.0
+                // -> 11.7.
                 constexpr int GQ = CX ? 2 : 4;  // output columns per group
                 constexpr int NP = CX ? 2 : 1;  // parts per output column
                 const uint64_t nanb = 0x7FF8000000000000ull;
+                X96 xs[HALF];
 #pragma unroll
+                for (int j = 0; j < HALF; ++j) xs[j] = words(j);
+#pragma unroll 1
                 for (int j0 = 0; j0 < NCOL; j0 += GQ) {
                     uint64_t bits[GQ][NP];
                     int Eq[GQ];
-                    bool slow = false;
+                    bool plain = true, fit = true;
 #pragma unroll
                     for (int q2 = 0; q2 < GQ; ++q2) {
-                        const int bc = __shfl_sync(0xffffffffu, lexp, j0 + q2);
-                        Eq[q2] = erow + (bc == 0 ? -1022 : bc - 1022) - W * (S + 1);
+                        Eq[q2] = erow + __shfl_sync(0xffffffffu, lexp, j0 + q2);
+                        plain = plain && x96_plain_exponent(Eq[q2]);
 #pragma unroll
-                        for (int pp = 0; pp < NP; ++pp) {
-                            const int j = NP * (j0 + q2) + pp;
-                            bits[q2][pp] = x96_ldexp_bits_fast(w0[j], w1[j], w2[j], Eq[q2], slow);
-                        }
+                        for (int pp = 0; pp < NP; ++pp) fit = fit && x96_is_64(xs[NP * q2 + pp].w1, xs[NP * q2 + pp].w2);
                     }
-                    if (slow) {
+                    if (__all_sync(0xffffffffu, plain && fit)) {
 #pragma unroll
                         for (int q2 = 0; q2 < GQ; ++q2)
 #pragma unroll
                             for (int pp = 0; pp < NP; ++pp) {
-                                const int j = NP * (j0 + q2) + pp;
-                                bits[q2][pp] =
-                                    (uint64_t)__double_as_longlong(x96_ldexp_rn_general(w0[j], w1[j], w2[j], Eq[q2]));
+                                const X96 &w = xs[NP * q2 + pp];
+                                bits[q2][pp] = x96_pack(x64_normalise(w.w0, w.w1), Eq[q2]);
+                            }
+                    } else if (__all_sync(0xffffffffu, plain)) {
+#pragma unroll
+                        for (int q2 = 0; q2 < GQ; ++q2)
+#pragma unroll
+                            for (int pp = 0; pp < NP; ++pp) {
+                                const X96 &w = xs[NP * q2 + pp];
+                                bits[q2][pp] = x96_pack(x96_normalise(w.w0, w.w1, w.w2), Eq[q2]);
+                            }
+                    } else {
+#pragma unroll
+                        for (int q2 = 0; q2 < GQ; ++q2)
+#pragma unroll
+                            for (int pp = 0; pp < NP; ++pp) {
+                                const X96 &w = xs[NP * q2 + pp];
+                                const double v = x96_ldexp_rn(w.w0, w.w1, w.w2, Eq[q2]);
+                                bits[q2][pp] = Eq[q2] > OZ_NAN_EXP / 2 ? nanb : (uint64_t)__double_as_longlong(v);
                             }
                     }
 #pragma unroll
                     for (int q2 = 0; q2 < GQ; ++q2) {
-                        const int jj = j0 + q2;
-                        const int64_t coff = __shfl_sync(0xffffffffu, lcoff, jj);
-                        const int bc = __shfl_sync(0xffffffffu, lexp, jj);
-                        if (!row_ok || bc < 0) continue;
-                        const int64_t off = rowoff + coff;
-                        const bool bad = badrow || bc == 0x7FF;
-                        const double v0 = __longlong_as_double((long long)(bad ? nanb : bits[q2][0]));
+                        const int64_t off = rowoff + __shfl_sync(0xffffffffu, lcoff, j0 + q2);
+                        if (!row_ok || !(cols >> (j0 + q2) & 1u)) continue;
+                        const double v0 = __longlong_as_double((long long)bits[q2][0]);
                         if constexpr (CX) {
-                            const double v1 = __longlong_as_double((long long)(bad ? nanb : bits[q2][NP - 1]));
+                            const double v1 = __longlong_as_double((long long)bits[q2][NP - 1]);
                             ((double2 *)Cl)[off] = make_double2(v0, v1);
                         } else {
                             ((double *)Cl)[off] = v0;
                         }
                     }
+#pragma unroll
+                    for (int j = 0; j + GQ * NP < HALF; ++j) xs[j] = xs[j + GQ * NP];
                 }
             } else {
 #pragma unroll
                 for (int jj = 0; jj < NCOL; ++jj) {
                     const int64_t coff = __shfl_sync(0xffffffffu, lcoff, jj);
-                    const int bc = __shfl_sync(0xffffffffu, lexp, jj);
-                    if (!row_ok || bc < 0) continue;
+                    if (!row_ok || !(cols >> jj & 1u)) continue;
                     const int j = CX ? 2 * jj : jj;
                     const int64_t off = rowoff + coff;
                     if (CX) ((float2 *)Cl)[off] = make_float2(accf[j], accf[j + 1]);
@@ -805,6 +973,14 @@ __device__ __forceinline__ void oz_gemm_body(const Src &src) {
                 }
             }
         }
+    };
+    if (warp == 0) {
+        produce();
+    } else if (warp == 1 || (NI == 2 && warp == OZ_ISSUER2_WARP)) {
+        if constexpr (WIDE) issue_wide();
+        else issue_narrow();
+    } else if (warp < 2 + OZ_EPI_WARPS) {
+        epilogue();
     }
     tc_fence_before();
     __syncthreads();
@@ -862,11 +1038,14 @@ inline int set_smem_attr(K kern, int smem, std::atomic<bool> (&done)[OZ_MAX_DEVI
     return fail(MGB_ERR_ARGUMENT, "unsupported slice count");
 
 // The contraction of `job`, on a persistent grid (one CTA per SM, each
-// walking its share of the units).
+// walking its share of the units), in narrow tiles.
 int oz_launch_one(int S, bool exact, bool cx, const OzJob &job, int64_t units, cudaStream_t s);
 // The contraction of `job` with the slice count that the device chose (exact
-// form; nothing when that is 0, the plain form).
+// form; nothing when that is 0, the plain form, or not in job.cand).
 int oz_launch_any(bool cx, const OzAnyJob &job, int64_t units, cudaStream_t s);
+// In wide tiles, with the count that the device chose (nothing unless it is in
+// job.cand) or job.S.
+int oz_launch_wide(bool cx, const OzAnyJob &job, int64_t units, cudaStream_t s);
 // Every contraction of a device table of one kernel variant.
 int oz_launch_table(int S, bool exact, bool cx, const OzJob *jobs, const int64_t *start, int njobs, int64_t units,
                     cudaStream_t s);

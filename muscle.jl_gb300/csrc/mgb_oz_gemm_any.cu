@@ -12,16 +12,16 @@ namespace mgb {
 // of the fixed kernels; registers and shared memory are the largest of them,
 // which the one CTA per SM has anyway.
 template <bool CX>
-__global__ void __launch_bounds__(OZ_THREADS, 1) k_oz_gemm_any(const __grid_constant__ OzAnyJob job) {
+__global__ void __launch_bounds__(oz_threads(false), 1) k_oz_gemm_any(const __grid_constant__ OzAnyJob job) {
     const int S = *job.a.sel;
     if (S == 0 || !(job.cand & (1u << S))) return;  // the plain form
     switch (S) {
-    case 3: oz_gemm_body<3, true, CX>(OzChosenJob<3>{&job}); return;
-    case 4: oz_gemm_body<4, true, CX>(OzChosenJob<4>{&job}); return;
-    case 5: oz_gemm_body<5, true, CX>(OzChosenJob<5>{&job}); return;
-    case 6: oz_gemm_body<6, true, CX>(OzChosenJob<6>{&job}); return;
-    case 7: oz_gemm_body<7, true, CX>(OzChosenJob<7>{&job}); return;
-    case 8: oz_gemm_body<8, true, CX>(OzChosenJob<8>{&job}); return;
+    case 3: oz_gemm_body<3, true, CX, false>(OzChosenJob<3>{&job}); return;
+    case 4: oz_gemm_body<4, true, CX, false>(OzChosenJob<4>{&job}); return;
+    case 5: oz_gemm_body<5, true, CX, false>(OzChosenJob<5>{&job}); return;
+    case 6: oz_gemm_body<6, true, CX, false>(OzChosenJob<6>{&job}); return;
+    case 7: oz_gemm_body<7, true, CX, false>(OzChosenJob<7>{&job}); return;
+    case 8: oz_gemm_body<8, true, CX, false>(OzChosenJob<8>{&job}); return;
     }
 }
 static_assert(sizeof(OzAnyJob) <= 4096, "kernel parameters");
@@ -34,7 +34,7 @@ static int launch_any_t(const OzAnyJob &job, int64_t units, cudaStream_t s) {
     static std::atomic<bool> attr_set[OZ_MAX_DEVICES];
     if (int st = set_smem_attr(kern, smem, attr_set)) return st;
     const unsigned grid = (unsigned)std::min<int64_t>(units, sm_count());
-    kern<<<grid, OZ_THREADS, smem, s>>>(job);
+    kern<<<grid, oz_threads(false), smem, s>>>(job);
     MGB_CUDA_CHECK(cudaGetLastError());
     return MGB_OK;
 }

@@ -8,8 +8,8 @@ namespace mgb {
 // A single contraction: its job in the parameter space (the tensor maps
 // must lie in param, const or global memory for TMA).
 template <int S, bool EXACT, bool CX>
-__global__ void __launch_bounds__(OZ_THREADS, 1) k_oz_gemm(const __grid_constant__ OzJob job) {
-    oz_gemm_body<S, EXACT, CX>(OzOneJob{&job});
+__global__ void __launch_bounds__(oz_threads(false), 1) k_oz_gemm(const __grid_constant__ OzJob job) {
+    oz_gemm_body<S, EXACT, CX, false>(OzOneJob{&job});
 }
 
 template <int S, bool EXACT, bool CX>
@@ -19,7 +19,7 @@ static int launch_gemm_t(const OzJob &job, int64_t units, cudaStream_t s) {
     static std::atomic<bool> attr_set[OZ_MAX_DEVICES];
     if (int st = set_smem_attr(kern, smem, attr_set)) return st;
     const unsigned grid = (unsigned)std::min<int64_t>(units, sm_count());
-    kern<<<grid, OZ_THREADS, smem, s>>>(job);
+    kern<<<grid, oz_threads(false), smem, s>>>(job);
     MGB_CUDA_CHECK(cudaGetLastError());
     return MGB_OK;
 }

@@ -8,9 +8,9 @@ namespace mgb {
 
 // A group: every bucket of one kernel variant in one persistent launch.
 template <int S, bool EXACT, bool CX>
-__global__ void __launch_bounds__(OZ_THREADS, 1)
+__global__ void __launch_bounds__(oz_threads(false), 1)
     k_oz_gemm_grouped(const OzJob *__restrict__ jobs, const int64_t *__restrict__ start, int njobs) {
-    oz_gemm_body<S, EXACT, CX>(OzJobTable{jobs, start, njobs});
+    oz_gemm_body<S, EXACT, CX, false>(OzJobTable{jobs, start, njobs});
 }
 
 template <int S, bool EXACT, bool CX>
@@ -20,7 +20,7 @@ static int launch_grouped_t(const OzJob *jobs, const int64_t *start, int njobs, 
     static std::atomic<bool> attr_set[OZ_MAX_DEVICES];
     if (int st = set_smem_attr(kern, smem, attr_set)) return st;
     const unsigned grid = (unsigned)std::min<int64_t>(units, sm_count());
-    kern<<<grid, OZ_THREADS, smem, s>>>(jobs, start, njobs);
+    kern<<<grid, oz_threads(false), smem, s>>>(jobs, start, njobs);
     MGB_CUDA_CHECK(cudaGetLastError());
     return MGB_OK;
 }

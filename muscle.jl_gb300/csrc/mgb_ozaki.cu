@@ -601,15 +601,6 @@ __device__ __forceinline__ uint32_t oz_digit_pair(uint64_t u0, uint64_t u1) {
     const __half2 d = __hsub2(*reinterpret_cast<const __half2 *>(&w), *reinterpret_cast<const __half2 *>(&k));
     return *reinterpret_cast<const uint32_t *>(&d);
 }
-// f(integral_constant<int, s>) for s = 0 .. N-1, unrolled at compile time.
-template <int N, int s = 0, typename F>
-__device__ __forceinline__ void oz_static_for(F &&f) {
-    if constexpr (s < N) {
-        f(std::integral_constant<int, s>{});
-        oz_static_for<N, s + 1>(f);
-    }
-}
-
 // Three bf16 pieces of two floats: x = hi + mid + lo (to ~2^-24 relative).
 __device__ __forceinline__ void bf3_pairs(float x0, float x1, uint32_t (&p)[3]) {
 #pragma unroll
@@ -955,33 +946,55 @@ void ozaki_orient(ContractionPlan &p) {
 // slice count (all exact tiles are equally wide).
 constexpr int OZ_SPLIT_WAVES = 2;
 constexpr double OZ_SPLIT_FIXED = 2.0, OZ_SPLIT_EACH = 0.4, OZ_SPLIT_WAVE = 8.0, OZ_SPLIT_GAIN = 1.0;
-constexpr double oz_kb_us(bool exact) { return exact ? 0.6 : 0.4; }
-static uint64_t oz_part_bytes(bool exact) {
-    return (uint64_t)OZ_BM * oz_bn(exact ? 8 : 3, exact) * (exact ? 12 : 8);
+constexpr double oz_kb_us(bool exact, bool wide) { return wide ? 1.21 : exact ? 0.6 : 0.4; }
+// Wide or narrow tiles (see oz_gemm_body): the faster under these times (us,
+// S = 6, every SM busy): a k block 0.69 narrow and 1.21 wide, a launch 8 and
+// 25 (the wide readout's code, and the first chunk's MMAs, which nothing
+// overlaps), a wave of wide tiles 4 more; wide ones only if they save
+// OZ_WIDE_GAIN. Measured wide / narrow for 128 x 64 tiles x k blocks, us:
+// 152 x 128 184 / 182, 304 x 64 188 / 170, 608 x 32 192 / 165, 608 x 128
+// 662 / 700, 2432 x 64 1340 / 1396, 72 x 4096 (cut in two) 2600 / 3240,
+// 8192 x 256 16870 / 18620. With 3 slices wide tiles win a little earlier (152 x
+// 128 94 / 98).
+// The rule sees shapes only.
+constexpr uint32_t kWideCounts = 1u << 3 | 1u << 6;  // as a mask
+static_assert(oz_wide(3) && oz_wide(6) && !oz_wide(4) && !oz_wide(5) && !oz_wide(7) && !oz_wide(8), "kWideCounts");
+constexpr double OZ_KB_NARROW = 0.69, OZ_LAUNCH_NARROW = 8.0, OZ_LAUNCH_WIDE = 25.0, OZ_WAVE_WIDE = 4.0, OZ_WIDE_GAIN = 0.97;
+static uint64_t oz_part_bytes(bool exact, bool wide) {
+    return (uint64_t)OZ_BM * oz_bn(exact ? 8 : 3, exact, wide) * (exact ? 12 : 8);
 }
-// Sets the plan's split; returns the number of its units (0: no tile is split).
-static int64_t oz_split(ContractionPlan &p) {
-    const int64_t bn = oz_bn(p.slices, p.form == MGB_FORM_OZAKI);
+// The plan's tiling with narrow or wide tiles; `units` of its split tiles (0:
+// none is split) and the GEMM's time in us under the rule's model.
+static OzTiling oz_tiling(const ContractionPlan &p, bool wide, int64_t &units, double &us) {
+    const bool exact = p.form == MGB_FORM_OZAKI;
+    const int64_t bn = oz_bn(p.slices, exact, wide), sms = sm_count();
     const int64_t tiles = ((p.m_e + OZ_BM - 1) / OZ_BM) * ((p.n_e + bn - 1) / bn) * p.L;
-    const int64_t nkb = (p.k_e + OZ_BK - 1) / OZ_BK, sms = sm_count(), tail = tiles % sms;
-    p.split_full = tiles;
-    p.splits = 1;
-    p.split_kbs = 0;
-    if (tail == 0 || nkb > INT32_MAX / 2) return 0;
-    const double kb = oz_kb_us(p.form == MGB_FORM_OZAKI);
-    double best = nkb * kb - OZ_SPLIT_GAIN;
-    for (int64_t s = 2; s <= OZ_SPLIT_WAVES * sms / tail && s <= nkb; ++s) {
+    const int64_t nkb = (p.k_e + OZ_BK - 1) / OZ_BK, tail = tiles % sms;
+    const double kb = oz_kb_us(exact, wide);
+    OzTiling r;
+    r.full = tiles;
+    units = 0;
+    const double full_kb = exact && !wide ? OZ_KB_NARROW : kb;
+    const int64_t whole = tiles / sms;
+    us = (wide ? OZ_LAUNCH_WIDE + OZ_WAVE_WIDE * (whole + (tail > 0)) : OZ_LAUNCH_NARROW) + full_kb * (double)(whole * nkb);
+    if (tail == 0) return r;
+    double best = nkb * kb - OZ_SPLIT_GAIN, last = full_kb * nkb;
+    for (int64_t s = 2; s <= OZ_SPLIT_WAVES * sms / tail && s <= nkb && nkb < INT32_MAX / 2; ++s) {
         const int64_t kbs = (nkb + s - 1) / s, waves = (tail * s + sms - 1) / sms;
         if ((s - 1) * kbs >= nkb) continue;  // an empty last unit
-        const double t = waves * kbs * kb + (waves - 1) * OZ_SPLIT_WAVE + OZ_SPLIT_FIXED + OZ_SPLIT_EACH * s;
+        const double over = (waves - 1) * OZ_SPLIT_WAVE + OZ_SPLIT_FIXED + OZ_SPLIT_EACH * s;
+        const double t = waves * kbs * kb + over;
         if (t < best) {
             best = t;
-            p.split_full = tiles - tail;
-            p.splits = (int32_t)s;
-            p.split_kbs = (int32_t)kbs;
+            last = waves * kbs * full_kb + over;
+            r.full = tiles - tail;
+            r.splits = (int32_t)s;
+            r.kbs = (int32_t)kbs;
         }
     }
-    return p.splits > 1 ? tail * p.splits : 0;
+    units = r.splits > 1 ? tail * r.splits : 0;
+    us += last;
+    return r;
 }
 
 void ozaki_setup(ContractionPlan &p) {
@@ -1026,18 +1039,34 @@ void ozaki_setup(ContractionPlan &p) {
         }
     }
     p.ws_min = off;
-    if (const int64_t units = oz_split(p)) {
+    // tilings, and room for the split tiles of those that may run
+    const bool exact = p.form == MGB_FORM_OZAKI;
+    int64_t units[2] = {0, 0};
+    double us[2];
+    p.tile[0] = oz_tiling(p, false, units[0], us[0]);
+    p.wide = false;
+    if (exact && (p.adaptive || oz_wide(S))) {
+        p.tile[1] = oz_tiling(p, true, units[1], us[1]);
+        p.wide = us[1] < us[0] * OZ_WIDE_GAIN;
+    }
+    uint64_t cnt = 0, part = 0;
+    for (int w = 0; w < (p.wide ? 2 : 1); ++w)
+        if (units[w]) {
+            cnt = std::max(cnt, (uint64_t)(units[w] / p.tile[w].splits) * OZ_EPI_WARPS * 4);
+            part = std::max(part, (uint64_t)units[w] * oz_part_bytes(exact, w));
+        }
+    if (part) {
         p.ws_cnt = off;
-        off = align256(off + units / p.splits * OZ_EPI_WARPS * 4);
+        off = align256(off + cnt);
         p.ws_part = off;
-        off = align256(off + units * oz_part_bytes(p.form == MGB_FORM_OZAKI));
+        off = align256(off + part);
     }
     p.ws_bytes = off;
 }
 
 // Counters of the split tiles (one per tile and epilogue warp).
 static int split_counters(const ContractionPlan &p) {
-    if (p.splits <= 1) return 0;
+    if (p.ws_bytes == p.ws_min) return 0;
     return (int)((p.ws_part - p.ws_cnt) / 4);  // with the padding between the two areas
 }
 
@@ -1231,12 +1260,13 @@ int ozaki_prepass(const ContractionPlan &p, const void *A, const void *B, void *
 
 // The GEMM's view of a plan whose slices lie in `ws`. `split`: the workspace
 // has room for the sums of split tiles (ws_bytes, not only ws_min).
-static int ozaki_shape(const ContractionPlan &p, void *C, void *ws, bool split, OzJobShape &job) {
+static int ozaki_shape(const ContractionPlan &p, void *C, void *ws, bool split, bool wide, OzJobShape &job) {
     const bool exact = p.form == MGB_FORM_OZAKI;
     uint8_t *w = (uint8_t *)ws;
     int32_t *status = device_status_ptr();
     if (!status) return fail(MGB_ERR_CUDA, "device status word unavailable");
-    const int bn = oz_bn(p.slices, exact);
+    const int bn = oz_bn(p.slices, exact, wide);
+    const OzTiling &tile = p.tile[wide ? 1 : 0];
     OzGemmArgs &a = job.a;
     a.M = p.M;
     a.Ne = p.n_e;
@@ -1261,21 +1291,23 @@ static int ozaki_shape(const ContractionPlan &p, void *C, void *ws, bool split, 
     a.full = (int64_t)job.tiles_n * job.tiles_m * job.L;
     a.splits = 1;
     a.kbs = a.nkb;
-    if (split && p.splits > 1) {
-        a.full = p.split_full;
-        a.splits = p.splits;
-        a.kbs = p.split_kbs;
+    if (split && tile.splits > 1) {
+        a.full = tile.full;
+        a.splits = tile.splits;
+        a.kbs = tile.kbs;
         a.cnt = (int32_t *)(w + p.ws_cnt);
         a.part = (uint32_t *)(w + p.ws_part);
     }
     return MGB_OK;
 }
 // The slice tensor maps and the band for S slices.
-static int ozaki_maps(const ContractionPlan &p, void *ws, int S, CUtensorMap *ta, CUtensorMap *tb, int32_t &band) {
+static int ozaki_maps(const ContractionPlan &p, void *ws, int S, bool wide, CUtensorMap *ta, CUtensorMap *tb,
+                      int32_t &band) {
     uint8_t *w = (uint8_t *)ws;
     int st;
     if ((st = make_map(ta, w + p.ws_a, p.k_e, p.m_e, p.L * S, p.kpad, OZ_BM, S))) return st;
-    if ((st = make_map(tb, w + p.ws_b, p.k_e, p.n_e, p.L * S, p.kpad, oz_bn(S, p.form == MGB_FORM_OZAKI), S))) return st;
+    if ((st = make_map(tb, w + p.ws_b, p.k_e, p.n_e, p.L * S, p.kpad, oz_bn(S, p.form == MGB_FORM_OZAKI, wide), S)))
+        return st;
     band = p.band;
     if (band <= 0) {
         band = OZ_GROUP_M;
@@ -1284,34 +1316,57 @@ static int ozaki_maps(const ContractionPlan &p, void *ws, int S, CUtensorMap *ta
     return MGB_OK;
 }
 // A job of slice count S (0: the plan's), run only when `sel` (nullable) holds S.
-static int ozaki_job(const ContractionPlan &p, void *C, void *ws, bool split, OzJob &job, int64_t &units, int S = 0,
+// In narrow tiles.
+static int ozaki_job(const ContractionPlan &p, void *C, void *ws, bool split, OzJob &job, int S = 0,
                      const int32_t *sel = nullptr) {
     std::memset(&job, 0, sizeof(job));
-    if (int st = ozaki_shape(p, C, ws, split, job)) return st;
+    if (int st = ozaki_shape(p, C, ws, split, false, job)) return st;
     job.a.sel = sel;
-    units = job.units();
-    return ozaki_maps(p, ws, S ? S : p.slices, &job.tmA, &job.tmB, job.band);
+    return ozaki_maps(p, ws, S ? S : p.slices, false, &job.tmA, &job.tmB, job.band);
+}
+
+// The job of every slice count in `cand`, of which `sel` (nullable) names the
+// one to run; without it cand is one count.
+static int ozaki_any_job(const ContractionPlan &p, void *C, void *ws, bool split, bool wide, uint32_t cand,
+                         const int32_t *sel, OzAnyJob &job) {
+    std::memset(&job, 0, sizeof(job));
+    if (int st = ozaki_shape(p, C, ws, split, wide, job)) return st;
+    job.a.sel = sel;
+    job.cand = cand;
+    for (int S = 3; S <= 8; ++S)
+        if (cand & (1u << S)) {
+            job.S = S;
+            if (int st = ozaki_maps(p, ws, S, wide, &job.tm[S - 3][0], &job.tm[S - 3][1], job.band[S - 3])) return st;
+        }
+    return MGB_OK;
 }
 
 int ozaki_gemm(const ContractionPlan &p, const void *A, const void *B, void *C, void *ws, bool split, cudaStream_t s) {
-    int64_t units = 0;
     const bool cx = is_complex(p.compute_dtype);
-    if (!p.adaptive) {
-        OzJob job;
-        if (int st = ozaki_job(p, C, ws, split, job, units)) return st;
-        return oz_launch_one(p.slices, p.form == MGB_FORM_OZAKI, cx, job, units, s);
-    }
-    // One launch, which reads the chosen count; with none chosen the plain form runs.
     OzAnyJob job;
-    std::memset(&job, 0, sizeof(job));
-    if (int st = ozaki_shape(p, C, ws, split, job)) return st;
+    if (!p.adaptive) {
+        if (p.wide) {
+            if (int st = ozaki_any_job(p, C, ws, split, true, 1u << p.slices, nullptr, job)) return st;
+            return oz_launch_wide(cx, job, job.units(), s);
+        }
+        OzJob one;
+        if (int st = ozaki_job(p, C, ws, split, one)) return st;
+        return oz_launch_one(p.slices, p.form == MGB_FORM_OZAKI, cx, one, one.units(), s);
+    }
+    // The kernels read the chosen count: one launch, or one for the counts
+    // that wide tiles hold and one for the others. With none chosen the plain
+    // form runs.
     const int32_t *sel = &stat_area(p, ws).st->sel;
-    job.a.sel = sel;
-    job.cand = p.cand_mask;
-    for (int S = 3; S <= 8; ++S)
-        if (p.cand_mask & (1u << S))
-            if (int st = ozaki_maps(p, ws, S, &job.tm[S - 3][0], &job.tm[S - 3][1], job.band[S - 3])) return st;
-    if (int st = oz_launch_any(cx, job, job.units(), s)) return st;
+    uint32_t narrow = p.cand_mask;
+    if (p.wide && (p.cand_mask & kWideCounts)) {
+        if (int st = ozaki_any_job(p, C, ws, split, true, p.cand_mask & kWideCounts, sel, job)) return st;
+        if (int st = oz_launch_wide(cx, job, job.units(), s)) return st;
+        narrow &= ~kWideCounts;
+    }
+    if (narrow) {
+        if (int st = ozaki_any_job(p, C, ws, split, false, narrow, sel, job)) return st;
+        if (int st = oz_launch_any(cx, job, job.units(), s)) return st;
+    }
     return launch_plain_gemm(p, A, B, C, s, sel);
 }
 
@@ -1373,15 +1428,14 @@ int ozaki_grouped_create(const std::vector<const ContractionPlan *> &plans, cons
             delete g;
             return fail(MGB_ERR_ARGUMENT, "grouped GEMM: plans of different kernel variants");
         }
-        int64_t t = 0;
         // an adaptive plan's job works only when its device choice is S
-        const int st = p.adaptive ? ozaki_job(p, nullptr, ws[i], true, host[i], t, S, &stat_area(p, ws[i]).st->sel)
-                                  : ozaki_job(p, nullptr, ws[i], true, host[i], t);
+        const int st = p.adaptive ? ozaki_job(p, nullptr, ws[i], true, host[i], S, &stat_area(p, ws[i]).st->sel)
+                                  : ozaki_job(p, nullptr, ws[i], true, host[i]);
         if (st) {
             delete g;
             return st;
         }
-        start[i + 1] = start[i] + t;
+        start[i + 1] = start[i] + host[i].units();
     }
     g->njobs = (int)plans.size();
     g->tiles = start.back();
@@ -1859,14 +1913,12 @@ int ozaki_batch_launch(const std::vector<OzBatchItem> &items, OzBatchBuffers *bu
             for (int S = 3; S <= 8; ++S) {
                 if (!(p.cand_mask & (1u << S))) continue;
                 OzJob job;
-                int64_t tiles;
-                if (int st = ozaki_job(p, it.C, it.ws, it.split, job, tiles, S, &a.st->sel)) return st;
+                if (int st = ozaki_job(p, it.C, it.ws, it.split, job, S, &a.st->sel)) return st;
                 gem[std::make_tuple(S, 1, cx ? 1 : 0)].push_back(job);
             }
         } else {
             OzJob job;
-            int64_t tiles;
-            if (int st = ozaki_job(p, it.C, it.ws, it.split, job, tiles)) return st;
+            if (int st = ozaki_job(p, it.C, it.ws, it.split, job)) return st;
             gem[std::make_tuple(exact ? p.slices : 3, exact ? 1 : 0, cx ? 1 : 0)].push_back(job);
         }
     }

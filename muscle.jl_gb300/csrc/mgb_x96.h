@@ -51,9 +51,8 @@ MGB_HD uint32_t x96_shl_funnel(uint32_t lo, uint32_t hi, int c) {
 // rounded to nearest, ties to even, including subnormal results and overflow
 // to infinity; X = 0 gives +0. Integer operations only: GB300 retires about
 // two FP64 operations per cycle per SM, and a short-K tile writes thousands
-// of outputs per CTA. This is the general routine with a branch per case;
-// the epilogue runs x96_ldexp_bits_fast and comes here only for subnormal
-// results.
+// of outputs per CTA. This is the general routine with a branch per case, for
+// subnormal results.
 MGB_HD double x96_ldexp_rn_general(uint32_t w0, uint32_t w1, uint32_t w2, int E) {
     const uint64_t neg = w2 >> 31;
     uint64_t lo = ((uint64_t)w1 << 32) | w0;
@@ -102,9 +101,7 @@ MGB_HD double x96_ldexp_rn_general(uint32_t w0, uint32_t w1, uint32_t w2, int E)
 // `slow` for a subnormal result, whose bits it does not compute. |X| is
 // normalised so that its leading one is bit 95 (whole words by selects, then
 // a funnel shift), which puts the 53-bit significand, the guard bit and the
-// sticky bits at fixed places. Without branches, the conversions of the
-// columns a thread writes are independent instruction streams that the
-// compiler interleaves.
+// sticky bits at fixed places.
 MGB_HD uint64_t x96_ldexp_bits_fast(uint32_t w0, uint32_t w1, uint32_t w2, int E, bool &slow) {
     const uint32_t neg = w2 >> 31, flip = 0u - neg;
     // |X| = (X ^ flip) + neg over 96 bits
@@ -145,6 +142,61 @@ MGB_HD double x96_ldexp_rn(uint32_t w0, uint32_t w1, uint32_t w2, int E) {
     bool slow = false;
     const uint64_t b = x96_ldexp_bits_fast(w0, w1, w2, E, slow);
     return slow ? x96_ldexp_rn_general(w0, w1, w2, E) : x96_bits_to_double(b);
+}
+
+// The same conversion in two steps for the exponents that leave every result
+// normal (or +0): a nonzero |X| lies in 1 .. 2^95, so E >= -1022 excludes
+// subnormals and E <= 927 overflow, after rounding too.
+MGB_HD bool x96_plain_exponent(int E) { return (unsigned)(E + 1022) <= 1022u + 927u; }
+
+// X as its sign, the position p of |X|'s leading one, and |X| shifted so that
+// the leading one is bit 63 of hi:lo, with every bit below bit 0 collapsed
+// into it. hi = 0 for X = 0 only.
+struct X96Norm {
+    uint32_t hi, lo, sign;  // sign: 0 or 2^31
+    int p;
+};
+MGB_HD X96Norm x96_normalise(uint32_t w0, uint32_t w1, uint32_t w2) {
+    const uint32_t neg = w2 >> 31, flip = 0u - neg;
+    uint32_t a0 = w0 ^ flip, a1 = w1 ^ flip, a2 = w2 ^ flip;
+    uint64_t t = (uint64_t)a0 + neg;
+    a0 = (uint32_t)t;
+    t = (uint64_t)a1 + (t >> 32);
+    a1 = (uint32_t)t;
+    a2 += (uint32_t)(t >> 32);
+    int top = 95;
+#pragma unroll
+    for (int r = 0; r < 2; ++r) {
+        const bool up = a2 == 0;
+        a2 = up ? a1 : a2;
+        a1 = up ? a0 : a1;
+        a0 = up ? 0u : a0;
+        top -= up ? 32 : 0;
+    }
+    const int c = x96_clz32(a2) & 31;  // a2 is zero only for X = 0
+    const uint32_t hi = x96_shl_funnel(a1, a2, c), lo = x96_shl_funnel(a0, a1, c);
+    return X96Norm{hi, lo | ((a0 << c) ? 1u : 0u), neg << 31, top - c};
+}
+// For X in the range of int64 (w2 is w1's sign): one word less to normalise,
+// and no bit falls below bit 0.
+MGB_HD bool x96_is_64(uint32_t w1, uint32_t w2) { return w2 == 0u - (w1 >> 31); }
+MGB_HD X96Norm x64_normalise(uint32_t w0, uint32_t w1) {
+    const uint64_t x = ((uint64_t)w1 << 32) | w0;
+    const uint64_t a = (w1 >> 31) ? 0 - x : x;
+    const uint32_t ah = (uint32_t)(a >> 32), al = (uint32_t)a;
+    const bool up = ah == 0;
+    const uint32_t hi = up ? al : ah, lo = up ? 0u : al;
+    const int c = x96_clz32(hi) & 31;
+    return X96Norm{x96_shl_funnel(lo, hi, c), lo << c, w1 & 0x80000000u, (up ? 31 : 63) - c};
+}
+// The float64 bits of a normalised X times 2^E, for a plain exponent E:
+// rounded to nearest, ties to even; a carry out of the significand bumps the
+// exponent field.
+MGB_HD uint64_t x96_pack(const X96Norm &n, int E) {
+    const uint32_t lo = (n.lo >> 11) | (n.hi << 21), hi = n.hi >> 11;  // 53 bits with the leading one
+    const uint32_t up = (n.lo & 0x7FFu) + (lo & 1u) > 0x400u;
+    const uint32_t top = n.hi ? (uint32_t)(n.p + E + 1022) << 20 : 0u;
+    return ((((uint64_t)(hi + top)) << 32) | lo) + up + ((uint64_t)n.sign << 32);
 }
 
 }  // namespace mgb
