@@ -6,6 +6,7 @@ symbol is absent, the import of the compute entry points raises.
 from __future__ import annotations
 
 import ctypes
+import functools
 import os
 import threading
 
@@ -144,6 +145,8 @@ def lib_path() -> str:
 def load(build_if_missing: bool = True):
     """Returns the loaded library, building it in-tree when it is absent."""
     global _lib
+    if _lib is not None:
+        return _lib
     with _lock:
         if _lib is not None:
             return _lib
@@ -217,3 +220,8 @@ def make_desc(dtype: int, modes, extents, strides):
     s = (ctypes.c_int64 * max(r, 1))(*strides)
     d = TensorDesc(dtype, r, m, e, s)
     return d, (m, e, s)
+
+
+# The same for tuples, the last ones kept and shared (so read only): operations
+# without a plan build two or three a call, 3 us each.
+kept_desc = functools.lru_cache(maxsize=4096)(make_desc)

@@ -40,7 +40,7 @@ class DomainCUDA(Domain):
 
 def domain(x) -> Domain:
     """Memory domain of an array or Tensor (src/Domain.jl:11-14)."""
-    data = getattr(x, "data", x)
+    data = x if isinstance(x, torch.Tensor) else getattr(x, "data", x)
     if isinstance(data, torch.Tensor) and data.is_cuda:
         return DomainCUDA()
     return DomainHost()

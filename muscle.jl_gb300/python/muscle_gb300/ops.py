@@ -17,7 +17,7 @@ import torch
 from . import _lib
 from ._lib import ArgumentError, check
 from .backend import Backend, DomainCUDA, choose_backend, register_rule
-from .tensor import Index, Tensor, empty_colmajor, intersect, nonunique, setdiff, union
+from .tensor import Index, Tensor, empty_colmajor, intersect, nonunique, setdiff, union, unique
 
 _DT = {torch.float32: _lib.F32, torch.float64: _lib.F64, torch.complex64: _lib.C32, torch.complex128: _lib.C64}
 _TORCH = {v: k for k, v in _DT.items()}
@@ -163,6 +163,8 @@ def unary_plan(x: torch.Tensor, ix, y: torch.Tensor, iy) -> Plan:
 
 
 def _stream_handle(dev) -> int:
+    if isinstance(dev, torch.device) and dev.index is not None:
+        return torch._C._cuda_getCurrentRawStream(dev.index)  # without a Stream object around it
     return torch.cuda.current_stream(dev).cuda_stream
 
 
@@ -277,9 +279,9 @@ class BackendGB300(Backend):
             raise ArgumentError("hadamard: inds(b) must be a subset of inds(a)")
         modes = _modes_for(a.inds)
         lib = _lib.load()
-        (ad, ka), (bd, kb), (cd, kc) = (_lib.make_desc(*_desc_args(a.data, a.inds, modes)),
-                                        _lib.make_desc(*_desc_args(b.data, b.inds, modes)),
-                                        _lib.make_desc(*_desc_args(c.data, c.inds, modes)))
+        (ad, ka), (bd, kb), (cd, kc) = (_lib.kept_desc(*_desc_args(a.data, a.inds, modes)),
+                                        _lib.kept_desc(*_desc_args(b.data, b.inds, modes)),
+                                        _lib.kept_desc(*_desc_args(c.data, c.inds, modes)))
         check(lib.mgb_hadamard(ctypes.byref(ad), ctypes.byref(bd), ctypes.byref(cd), a.data.data_ptr(),
                                b.data.data_ptr(), c.data.data_ptr(), _stream_handle(c.data.device)), lib)
         return c
@@ -443,19 +445,26 @@ def hadamard_(c: Tensor, a: Tensor, b: Tensor) -> Tensor:
     return c
 
 
+def _same_labels(xs, ys) -> bool:
+    """The same labels, each as often, in any order."""
+    if len(xs) != len(ys) or any(x not in ys for x in xs):
+        return False
+    return len(unique(xs)) == len(xs) or sorted(map(repr, xs)) == sorted(map(repr, ys))
+
+
 def permutedims(t: Tensor, perm) -> Tensor:
     """Device permutation by labels (src/Tensor.jl:316-319) through the
     permutation kernel; ``perm`` is a list of Index labels or positions."""
     if t.ndim == 0:
         return t
     labels = [t.inds[p] if isinstance(p, int) else (p if isinstance(p, Index) else Index(p)) for p in perm]
-    if sorted(map(repr, labels)) != sorted(map(repr, t.inds)):
+    if not _same_labels(labels, t.inds):
         raise ArgumentError("permutation must use every label once")
     _require_cuda(t.data)
     y = empty_colmajor([t.size(i) for i in labels], t.dtype, t.data.device)
     modes = _modes_for(t.inds)
-    (xd, kx) = _lib.make_desc(*_desc_args(t.data, t.inds, modes))
-    (yd, ky) = _lib.make_desc(*_desc_args(y, labels, modes))
+    (xd, kx) = _lib.kept_desc(*_desc_args(t.data, t.inds, modes))
+    (yd, ky) = _lib.kept_desc(*_desc_args(y, labels, modes))
     lib = _lib.load()
     check(lib.mgb_permute(ctypes.byref(xd), ctypes.byref(yd), t.data.data_ptr(), y.data_ptr(),
                           _stream_handle(y.device)), lib)
