@@ -1212,10 +1212,10 @@ def main():
     flops = plan.flops
     value = flops * ws * args.steps / (ms / 1e3) / 1e12
     # kernels of one adaptive step: the exponent scan, the statistics with the
-    # choice, the slicer, the tcgen05 GEMM of the chosen slice count and the
-    # plain DMMA candidate, which returns at once unless it was chosen (plus a
-    # memset)
-    launches_per_step = 5
+    # choice, the slicer, the tcgen05 GEMM in wide tiles and in narrow ones (the
+    # one without the chosen slice count returns at once) and the plain DMMA
+    # candidate, which does so too unless it was chosen (plus a memset)
+    launches_per_step = 6
 
     # kernel timing for the roofline: phase events around the GEMM launch
     lib.mgb_plan_set_timing(plan.handle, 1)
@@ -1306,7 +1306,7 @@ def main():
             "metric": METRIC, "value": value, "unit": "TFLOP/s", "n_gpus": ws, "steps": args.steps,
             "warmup": args.warmup, "ms_per_step": ms / args.steps, "higher_is_better": True, "scaling": "weak",
             "vs_baseline": None, "dtype": "c64", "data": "synthetic", "config": workload_config(n),
-            "form": f"ozaki, slice count {'adaptive' if plan.adaptive else 'fixed'}: S={S} (bf16 digits of "
+            "form": f"ozaki, slice count {'adaptive' if plan.adaptive else 'fixed'}: S={S} (Float16 digits of "
                     f"{8 if S <= 6 else 7} bits on tcgen05.mma kind::f16, exact int accumulation)",
             "adaptive_choice": choice,
             "rel_err": rel_err, "rel_err_reference": "plain FP64 DMMA result on the same inputs",
@@ -1322,7 +1322,7 @@ def main():
                     "result_matches_device_run": e2e_ok, "phases": e2e_phases},
             "roofline": {"bound": "tensor", "achieved": achieved, "peak": bf16_peak, "unit": "TFLOP/s",
                          "frac": achieved / bf16_peak, "traffic": traffic, "peak_kind": f"bf16 dense burst ({peak_kind})",
-                         "kernel": "k_oz_gemm", "kernel_ms": gemm_ms, "prepass_ms": prepass_ms,
+                         "kernel": "k_oz_gemm_wide" if S in (3, 6) else "k_oz_gemm_any", "kernel_ms": gemm_ms, "prepass_ms": prepass_ms,
                          "prepass_bytes": prepass_bytes, "prepass_gbs": prepass_bytes / (prepass_ms / 1e3) / 1e9,
                          "prepass_frac_of_hbm": prepass_bytes / (prepass_ms / 1e3) / 1e9 / hbm_peak,
                          "work": f"2 x {pairs} slice pairs x M x 2N x 2K bf16 flops per launch"},

@@ -55,7 +55,7 @@ typedef enum mgb_dtype {
 typedef enum mgb_form {
     MGB_FORM_AUTO = 0,   /* OZAKI for F64/C64 results, BF16X3 for F32/C32        */
     MGB_FORM_PLAIN = 1,  /* native arithmetic: FP64 DMMA / FP32 FFMA              */
-    MGB_FORM_OZAKI = 2,  /* FP64/C64 as exact bf16 integer slices on tcgen05      */
+    MGB_FORM_OZAKI = 2,  /* FP64/C64 as exact Float16 integer slices on tcgen05   */
     MGB_FORM_BF16X3 = 3  /* FP32/C32 as 3-piece bf16 split products on tcgen05    */
 } mgb_form;
 

@@ -49,6 +49,8 @@
 //   warps 2..9   epilogue: tcgen05.ld 32x32b.x16 per group and column half
 //                from the bank the MMAs are not writing, then tcgen05.st of
 //                zeros into what was read.
+// Long contractions with 3 or 6 slices run in 128 x 64 tiles with one bank and
+// one issuer (see oz_gemm_body in mgb_oz_gemm.h).
 // Every mbarrier wait is bounded; on timeout the CTA records
 // MGB_ERR_DEVICE_TIMEOUT in the device status word, drains its copies and
 // MMAs, frees TMEM and returns.
@@ -542,7 +544,7 @@ __global__ void __launch_bounds__(256) k_oz_stat(const __grid_constant__ StatArg
 // =============================================================================
 // Pre-pass 2: slices (OZAKI digits or BF16X3 pieces), permutation fused
 // =============================================================================
-// Output words (2 x bf16) of slice plane s: out[((l*S + s) * rows_e + row) * kw + word].
+// Output words (2 x 16 bits) of slice plane s: out[((l*S + s) * rows_e + row) * kw + word].
 //   MODE_REAL : row = r,        word w holds k = 2w, 2w+1
 //   MODE_CA   : row = r,        word k holds (re, im)           (A side)
 //   MODE_CB   : rows 2r, 2r+1,  word k holds (re, -im), (im, re) (B side)
