@@ -144,25 +144,70 @@ __device__ __forceinline__ double rsqrt_step(double x, double y0) {
     return fma(y0 * e, fma(e, 0.375, 0.5), y0);
 }
 
+__device__ __forceinline__ bool nonzero(double x) { return x != 0.0; }
+__device__ __forceinline__ bool nonzero(double2 x) { return x.x != 0.0 || x.y != 0.0; }
+
 // The rotation of a pair with squared norms a, b and inner product g =
 // w_p^H w_q: [w_p, w_q] <- [w_p, w_q] J, J = [[c, s e], [-s conj(e), c]],
 // e = g / |g|, makes w_p^H w_q vanish: t = s / c is the smaller root of
 // t^2 + d t - 1 with d = (b - a) / |g|. False when the pair is orthogonal
-// already (|g|^2 <= tol2 a b). Everything is scaled by the power of two that
-// brings the largest to [1, 2), so that squares stay in range whatever the
-// columns' magnitude. t has a relative error near 1e-13 (a float estimate and
-// one Newton step); c = 1 / sqrt(1 + t^2) makes J unitary for any t.
+// already (|g|^2 <= tol2 a b). t has a relative error near 1e-13 (a float
+// estimate and one Newton step); c = 1 / sqrt(1 + t^2) makes J unitary for any
+// t. This one for norms and inner products anywhere in the range of doubles, and
+// however far apart: g, a and b in the product, and the difference are each
+// scaled by the power of two that brings them near 1 and the powers kept as
+// integers; subnormal ones are multiplied by 2^512 first.
+template <typename T>
+__device__ __forceinline__ bool rotation_far(double a, double b, T g, double tol2, double &c, T &se, T &sec) {
+    int ea = dexp(a), eb = dexp(b), eg = dexp_max(g), be = max(max(ea, eb), eg);
+    if (be == 0x7FF || !nonzero(g)) return false;
+    if (be < 1500) {
+        constexpr double up = 1.3407807929942597e154;  // 2^512
+        a *= up;
+        b *= up;
+        g = sscale(g, up);
+        ea = dexp(a), eb = dexp(b), eg = dexp_max(g), be = max(max(ea, eb), eg);
+    }
+    if (eg == 0) return false;
+    g = dscale(g, 1023 - eg);
+    const double g2 = abs2(g);  // 1 .. 8
+    const int ab = ea + eb - 2 * eg;  // the exponent of a b / |g|^2
+    if (ea != 0 && eb != 0 &&
+        (ab > 300 || !(g2 > dscale(tol2 * (dscale(a, 1023 - ea) * dscale(b, 1023 - eb)), ab))))
+        return false;
+    const int ge = dexp(g2), k = (ge - 1023) >> 1;
+    const double ig = rsqrt_step(g2, f2d(f32_rsqrt(d2f(g2, 2 * k)), -k));
+    double d = (dscale(b, 1023 - be) - dscale(a, 1023 - be)) * ig;  // times 2^(be - eg)
+    // beyond 2^30, t is 1 / d to double precision: of d's mantissa, then scaled
+    const int e0 = dexp(d), de = e0 - 1023 + be - eg;
+    const bool far = e0 != 0 && de > 30;
+    d = dscale(d, far ? 1023 - e0 : be - eg);
+    const double ad = fabs(d);
+    const float df = d2f(ad, 0);
+    const float tf = far ? f32_rcp(df) : 2.f * f32_rcp(df + f32_sqrt(fmaf(df, df, 4.f)));
+    const float rf = far ? tf : f32_rcp(fmaf(2.f, tf, df));
+    const float cf = far ? 1.f : f32_rsqrt(fmaf(tf, tf, 1.f));
+    const double t0 = f2d(tf, 0);
+    double t = fma(-fma(t0, far ? ad : t0 + ad, -1.0), f2d(rf, 0), t0);
+    t = copysign(far ? dscale(t, -de) : t, d);
+    c = rsqrt_step(fma(t, t, 1.0), f2d(cf, 0));
+    se = sscale(g, c * t * ig);
+    sec = sscale(sconj(se), -1.0);
+    return true;
+}
+// The usual case: everything normal and within 2^400 of the largest, by whose
+// power of two all is scaled, so that squares stay in range.
 template <typename T>
 __device__ __forceinline__ bool rotation(double a, double b, T g, double tol2, double &c, T &se, T &sec) {
-    const int be = max(max(dexp(a), dexp(b)), dexp_max(g));
+    const int ea = dexp(a), eb = dexp(b), eg = dexp_max(g), be = max(max(ea, eb), eg), le = min(min(ea, eb), eg);
+    if (be == 0x7FF || le < 60 || be - le > 400) return rotation_far<T>(a, b, g, tol2, c, se, sec);
     const int sh = 1023 - be;
     a = dscale(a, sh);
     b = dscale(b, sh);
     g = dscale(g, sh);
     const double g2 = abs2(g);
-    const int ge = dexp(g2);
-    if (be == 0x7FF || ge == 0 || !(g2 > tol2 * (a * b))) return false;
-    const int k = (ge - 1023) >> 1;
+    if (!(g2 > tol2 * (a * b))) return false;
+    const int k = (dexp(g2) - 1023) >> 1;
     const double ig = rsqrt_step(g2, f2d(f32_rsqrt(d2f(g2, 2 * k)), -k));
     const double d = (b - a) * ig, ad = fabs(d);
     // beyond 2^30, t is 1 / d to double precision
