@@ -210,8 +210,8 @@ struct OzGemmArgs {
     const int32_t *sel;    // adaptive choice (nullable): run only when it holds S
     // Work units: the first `full` tiles are one unit each, every tile after
     // them is `splits` units of `kbs` k blocks (see oz_split). A split tile's
-    // units leave their sums in `part` and count in `cnt`; the last one adds
-    // them up and writes the outputs.
+    // units leave their sums in `part` and count in `cnt` (zero before and
+    // after); the last one adds them up and writes the outputs.
     int32_t splits, kbs;
     int64_t full;
     uint32_t *part;
@@ -382,14 +382,19 @@ __device__ __forceinline__ uint4 *oz_part_at(uint32_t *part, int unit, int w) {
     return (uint4 *)part + (((int64_t)unit * OZ_EPI_WARPS + w) * (NW / 4)) * 32 + threadIdx.x % 32;
 }
 // Publishes this warp's share and counts it; true for the warp that finds all
-// `splits` shares of its tile published. Nobody waits for anybody.
+// `splits` shares of its tile published, which sets the counter back to zero:
+// the GEMM may run again on the same slices. Nobody waits for anybody.
 __device__ __forceinline__ bool oz_part_last(int32_t *cnt, int tile, int w, int splits) {
     __threadfence();
     __syncwarp();
     int old = 0;
-    if (threadIdx.x % 32 == 0) old = atomicAdd(cnt + tile * OZ_EPI_WARPS + w, 1);
+    int32_t *c = cnt + tile * OZ_EPI_WARPS + w;
+    if (threadIdx.x % 32 == 0) old = atomicAdd(c, 1);
     const bool last = __shfl_sync(0xffffffffu, old, 0) == splits - 1;
-    if (last) __threadfence();
+    if (last) {
+        if (threadIdx.x % 32 == 0) *c = 0;
+        __threadfence();
+    }
     return last;
 }
 
