@@ -293,8 +293,10 @@ static UnarySplit unary_split(const UnaryPlan &p, bool ws) {
     const bool out_contig = p.go.n > 0 && std::llabs(p.go.str[0][0]) == 1 && p.go.ext[0] > 1;
     UnarySplit s;
     s.lanes = 1;
-    if (red_contig ? p.R >= 32 : p.R >= 64 && !out_contig) s.lanes = p.R >= 256 ? 32 : p.R >= 128 ? 16 : p.R >= 64 ? 8 : 4;
+    s.split = false;
     s.parts = 1;
+    if (p.O == 0) return s;  // nothing to share
+    if (red_contig ? p.R >= 32 : p.R >= 64 && !out_contig) s.lanes = p.R >= 256 ? 32 : p.R >= 128 ? 16 : p.R >= 64 ? 8 : 4;
     s.split = p.O * s.lanes < kUnaryThreadsWanted / 2 && p.R >= (s.lanes > 1 ? 1024 : 16);
     if (s.split && ws) {
         const int64_t units = s.lanes > 1 ? p.O : (p.O + 31) / 32;
