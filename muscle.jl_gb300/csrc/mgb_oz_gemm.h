@@ -374,6 +374,10 @@ __device__ __forceinline__ OzUnit oz_unit(const OzJobShape &J, int64_t local, in
     return u;
 }
 
+// The compensation of a sum that overflowed is not a number, while the sum is
+// an infinity that the next addition keeps: zero then, else the bits of c.
+__device__ __forceinline__ uint32_t finite_bits(float c) { return fabsf(c) <= 3.402823466e38f ? __float_as_uint(c) : 0u; }
+
 // ---- sums of a split tile ------------------------------------------------------
 // An epilogue warp's share of a unit: NW words per lane, as 16-byte vectors
 // of consecutive lanes.
@@ -862,9 +866,8 @@ __device__ __forceinline__ void oz_gemm_body(const Src &src) {
                         __stcg(mine + (j0 / 4) * 32,
                                make_uint4(__float_as_uint(accf[j0]), __float_as_uint(accf[j0 + 1]),
                                           __float_as_uint(accf[j0 + 2]), __float_as_uint(accf[j0 + 3])));
-                        __stcg(mine + ((HALF + j0) / 4) * 32,
-                               make_uint4(__float_as_uint(comp[j0]), __float_as_uint(comp[j0 + 1]),
-                                          __float_as_uint(comp[j0 + 2]), __float_as_uint(comp[j0 + 3])));
+                        __stcg(mine + ((HALF + j0) / 4) * 32, make_uint4(finite_bits(comp[j0]), finite_bits(comp[j0 + 1]),
+                                                                         finite_bits(comp[j0 + 2]), finite_bits(comp[j0 + 3])));
                     }
                 }
                 if (!oz_part_last(args.cnt, u.part / args.splits, w, args.splits)) continue;
