@@ -146,6 +146,7 @@ struct ContractionPlan {
     // workspace layout (byte offsets)
     uint64_t ws_cnt = 0, ws_part = 0;  // counters and sums of split tiles
     OzTiling tile[2];   // narrow and wide tiles of the emulated GEMM
+    int32_t sum_kb = 0; // BF16X3: k blocks per partial sum of every tile (0: one sum)
     bool wide = false;  // run in wide tiles where the slice count has them (not in a group)
     uint64_t ws_a = 0, ws_b = 0, ws_scale_a = 0, ws_scale_b = 0;
     int64_t kpad = 0;      // padded embedded K of the slice buffers

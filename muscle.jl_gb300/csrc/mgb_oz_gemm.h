@@ -132,6 +132,15 @@ __device__ __forceinline__ void tc_st16_zero(uint32_t taddr) {
         "r"(0u)
         : "memory");
 }
+// stores 16 consecutive columns of this warp's 32 lanes (no wait)
+__device__ __forceinline__ void tc_st16(uint32_t taddr, const float (&v)[16]) {
+    asm volatile(
+        "tcgen05.st.sync.aligned.32x32b.x16.b32 [%0], "
+        "{%1,%2,%3,%4,%5,%6,%7,%8,%9,%10,%11,%12,%13,%14,%15,%16};" ::"r"(taddr),
+        "f"(v[0]), "f"(v[1]), "f"(v[2]), "f"(v[3]), "f"(v[4]), "f"(v[5]), "f"(v[6]), "f"(v[7]), "f"(v[8]),
+        "f"(v[9]), "f"(v[10]), "f"(v[11]), "f"(v[12]), "f"(v[13]), "f"(v[14]), "f"(v[15])
+        : "memory");
+}
 __device__ __forceinline__ void tc_wait_st() { asm volatile("tcgen05.wait::st.sync.aligned;" ::: "memory"); }
 // NC consecutive columns (a multiple of 16), then wait for the loads
 template <int NC>
@@ -213,6 +222,9 @@ struct OzGemmArgs {
     // units leave their sums in `part` and count in `cnt` (zero before and
     // after); the last one adds them up and writes the outputs.
     int32_t splits, kbs;
+    // BF16X3: chunks per partial sum of a whole tile (0: one sum), those of the
+    // units that it would be cut into (see oz_sum_blocks)
+    int32_t fold;
     int64_t full;
     uint32_t *part;
     int32_t *cnt;
@@ -375,8 +387,15 @@ __device__ __forceinline__ OzUnit oz_unit(const OzJobShape &J, int64_t local, in
 }
 
 // The compensation of a sum that overflowed is not a number, while the sum is
-// an infinity that the next addition keeps: zero then, else the bits of c.
-__device__ __forceinline__ uint32_t finite_bits(float c) { return fabsf(c) <= 3.402823466e38f ? __float_as_uint(c) : 0u; }
+// an infinity that the next addition keeps: zero then, else c.
+__device__ __forceinline__ float finite_comp(float c) { return fabsf(c) <= 3.402823466e38f ? c : 0.f; }
+// Adds a partial sum x with its compensation c to a compensated sum (BF16X3);
+// the parts of a tile always in the order of k.
+__device__ __forceinline__ void add_part(float &sum, float &comp, float x, float c) {
+    const float t = x - (c + comp), s = sum + t;
+    comp = (s - sum) - t;
+    sum = s;
+}
 
 // ---- sums of a split tile ------------------------------------------------------
 // An epilogue warp's share of a unit: NW words per lane, as 16-byte vectors
@@ -443,6 +462,8 @@ __device__ __forceinline__ void oz_gemm_body(const Src &src) {
     constexpr int HALF = BN / 2;     // columns per group read by one epilogue warp
     constexpr int TCOLS = oz_tmem_cols(S);
     constexpr int BANK = TCOLS / 2;  // TMEM column offset of the second bank
+    constexpr int SUMS = BN * S;  // BF16X3: first free TMEM column of a bank
+    static_assert(EXACT || SUMS + BN <= BANK, "BF16X3: two sums per column beside the banks");
     static_assert(NST >= 2, "need at least two pipeline stages");
     static_assert(WIDE ? BN * S <= TCOLS : BN * S <= BANK, "the accumulators must fit in TMEM");
     static_assert(WIDE ? EXACT && oz_wide(S) : BN * S <= 256, "one MMA covers at most 256 columns");
@@ -743,7 +764,8 @@ __device__ __forceinline__ void oz_gemm_body(const Src &src) {
             // output column, x0 + x1 2^32
             uint32_t x0[EXACT ? HALF : 1];
             int64_t x1[EXACT ? HALF : 1];
-            // BF16X3: Kahan-compensated float32 sum over the chunks
+            // BF16X3: Kahan-compensated float32 sum over the chunks (of a part)
+            int left = args.fold;  // chunks to the end of the part
             float accf[EXACT ? 1 : HALF], comp[EXACT ? 1 : HALF];
 #pragma unroll
             for (int j = 0; j < HALF; ++j) {
@@ -838,6 +860,40 @@ __device__ __forceinline__ void oz_gemm_body(const Src &src) {
                     tc_fence_before();
                     __syncwarp();
                     if (lane == 0) mbar_arrive(smem_u32(acc_empty + bank));
+                    // A whole tile adds its parts as a cut one does: the sums so
+                    // far wait in the TMEM columns that the banks leave free.
+                    const bool last = c + 1 == nchunks;
+                    if (args.fold && u.part < 0 && (--left == 0 || last)) {
+                        left = args.fold;
+#pragma unroll
+                        for (int c2 = 0; c2 < HALF; c2 += 16) {
+                            float sum[16], cs[16];
+                            if (c >= args.fold) {
+                                uint32_t v0[16], v1[16];
+                                tc_ld16_issue(tbase + SUMS + c2, v0);
+                                tc_ld<16>(tbase + BANK + SUMS + c2, v1);
+#pragma unroll
+                                for (int j = 0; j < 16; ++j) {
+                                    sum[j] = __uint_as_float(v0[j]);
+                                    cs[j] = __uint_as_float(v1[j]);
+                                }
+                            } else {
+#pragma unroll
+                                for (int j = 0; j < 16; ++j) sum[j] = cs[j] = 0.f;
+                            }
+#pragma unroll
+                            for (int j = 0; j < 16; ++j) {
+                                add_part(sum[j], cs[j], accf[c2 + j], finite_comp(comp[c2 + j]));
+                                accf[c2 + j] = last ? sum[j] : 0.f;
+                                comp[c2 + j] = 0.f;
+                            }
+                            if (!last) {
+                                tc_st16(tbase + SUMS + c2, sum);
+                                tc_st16(tbase + BANK + SUMS + c2, cs);
+                            }
+                        }
+                        tc_wait_st();
+                    }
                 }
             }
             if (!ok) break;
@@ -866,8 +922,10 @@ __device__ __forceinline__ void oz_gemm_body(const Src &src) {
                         __stcg(mine + (j0 / 4) * 32,
                                make_uint4(__float_as_uint(accf[j0]), __float_as_uint(accf[j0 + 1]),
                                           __float_as_uint(accf[j0 + 2]), __float_as_uint(accf[j0 + 3])));
-                        __stcg(mine + ((HALF + j0) / 4) * 32, make_uint4(finite_bits(comp[j0]), finite_bits(comp[j0 + 1]),
-                                                                         finite_bits(comp[j0 + 2]), finite_bits(comp[j0 + 3])));
+                        __stcg(mine + ((HALF + j0) / 4) * 32,
+                               make_uint4(__float_as_uint(finite_comp(comp[j0])), __float_as_uint(finite_comp(comp[j0 + 1])),
+                                          __float_as_uint(finite_comp(comp[j0 + 2])),
+                                          __float_as_uint(finite_comp(comp[j0 + 3]))));
                     }
                 }
                 if (!oz_part_last(args.cnt, u.part / args.splits, w, args.splits)) continue;
@@ -902,12 +960,8 @@ __device__ __forceinline__ void oz_gemm_body(const Src &src) {
                             const uint4 x = __ldcg(p + (j0 / 4) * 32), y = __ldcg(p + ((HALF + j0) / 4) * 32);
                             const uint32_t xs[4] = {x.x, x.y, x.z, x.w}, ys[4] = {y.x, y.y, y.z, y.w};
 #pragma unroll
-                            for (int e = 0; e < 4; ++e) {
-                                const float t = __uint_as_float(xs[e]) - (__uint_as_float(ys[e]) + comp[j0 + e]);
-                                const float s2 = accf[j0 + e] + t;
-                                comp[j0 + e] = (s2 - accf[j0 + e]) - t;
-                                accf[j0 + e] = s2;
-                            }
+                            for (int e = 0; e < 4; ++e)
+                                add_part(accf[j0 + e], comp[j0 + e], __uint_as_float(xs[e]), __uint_as_float(ys[e]));
                         }
                     }
                 }

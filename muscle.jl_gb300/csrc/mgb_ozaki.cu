@@ -943,9 +943,8 @@ void ozaki_orient(ContractionPlan &p) {
 // readout waits for the first's sums to leave). One when none is shorter by
 // OZ_SPLIT_GAIN. E.g. one tile of 512 k blocks at S = 6: 279 us whole, 33 in
 // 32 units; 100 tiles of 128: 88 whole, 78 in 3 units; 75 tiles of 8: 16.4
-// whole, 17.9 in 2 units. The rule sees shapes only, so that a contraction is
-// cut the same way alone, in a group and in a served batch, and with every
-// slice count (all exact tiles are equally wide).
+// whole, 17.9 in 2 units. The bits of an exact result do not depend on the
+// cut.
 constexpr int OZ_SPLIT_WAVES = 2;
 constexpr double OZ_SPLIT_FIXED = 2.0, OZ_SPLIT_EACH = 0.4, OZ_SPLIT_WAVE = 8.0, OZ_SPLIT_GAIN = 1.0;
 constexpr double oz_kb_us(bool exact, bool wide) { return wide ? 1.21 : exact ? 0.6 : 0.4; }
@@ -965,6 +964,33 @@ constexpr double OZ_KB_NARROW = 0.69, OZ_LAUNCH_NARROW = 8.0, OZ_LAUNCH_WIDE = 2
 static uint64_t oz_part_bytes(bool exact, bool wide) {
     return (uint64_t)OZ_BM * oz_bn(exact ? 8 : 3, exact, wide) * (exact ? 12 : 8);
 }
+// BF16X3 sums round, so their bits depend on where a sum is cut, and that must
+// not depend on how the contraction is run: alone, as a member of a group or a
+// served batch, with the workspace for parts or without. So the parts of a sum
+// (k blocks in each, a multiple of the readout's chunk; 0: one sum) follow from
+// one batch entry's tiles and K, by the times above on OZ_SUM_SMS SMs, and a
+// tile adds them in the order of k whether its parts are units of their own
+// (oz_part_last) or it runs whole. Entries of a wave or more of tiles gain
+// little from a cut and have one sum.
+constexpr int64_t OZ_SUM_SMS = 152;
+static int32_t oz_sum_blocks(const ContractionPlan &p) {
+    const int64_t bn = oz_bn(3, false), chunk = oz_chunk(3, false);
+    const int64_t tiles = ((p.m_e + OZ_BM - 1) / OZ_BM) * ((p.n_e + bn - 1) / bn), nkb = (p.k_e + OZ_BK - 1) / OZ_BK;
+    if (tiles == 0 || tiles >= OZ_SUM_SMS || nkb >= INT32_MAX / 2) return 0;
+    const double kb = oz_kb_us(false, false);
+    double best = nkb * kb - OZ_SPLIT_GAIN;
+    int64_t kbs = 0;
+    for (int64_t most = 2; most <= OZ_SPLIT_WAVES * OZ_SUM_SMS / tiles; ++most) {
+        const int64_t c = ((nkb + most - 1) / most + chunk - 1) / chunk * chunk, s = (nkb + c - 1) / c;
+        const int64_t waves = (tiles * s + OZ_SUM_SMS - 1) / OZ_SUM_SMS;
+        const double t = waves * c * kb + (waves - 1) * OZ_SPLIT_WAVE + OZ_SPLIT_FIXED + OZ_SPLIT_EACH * s;
+        if (t < best) {
+            best = t;
+            kbs = s > 1 ? c : 0;
+        }
+    }
+    return (int32_t)kbs;
+}
 // The plan's tiling with narrow or wide tiles; `units` of its split tiles (0:
 // none is split) and the GEMM's time in us under the rule's model.
 static OzTiling oz_tiling(const ContractionPlan &p, bool wide, int64_t &units, double &us) {
@@ -981,6 +1007,18 @@ static OzTiling oz_tiling(const ContractionPlan &p, bool wide, int64_t &units, d
     us = (wide ? OZ_LAUNCH_WIDE + OZ_WAVE_WIDE * (whole + (tail > 0)) : OZ_LAUNCH_NARROW) + full_kb * (double)(whole * nkb);
     if (tail == 0) return r;
     double best = nkb * kb - OZ_SPLIT_GAIN, last = full_kb * nkb;
+    if (!exact) {  // cut into the parts of the sum, or not at all
+        if (p.sum_kb == 0) return r;
+        const int64_t s = (nkb + p.sum_kb - 1) / p.sum_kb, waves = (tail * s + sms - 1) / sms;
+        if (waves > 2 * OZ_SPLIT_WAVES ||
+            waves * p.sum_kb * kb + (waves - 1) * OZ_SPLIT_WAVE + OZ_SPLIT_FIXED + OZ_SPLIT_EACH * s >= best)
+            return r;
+        r.full = tiles - tail;
+        r.splits = (int32_t)s;
+        r.kbs = p.sum_kb;
+        units = tail * s;
+        return r;
+    }
     for (int64_t s = 2; s <= OZ_SPLIT_WAVES * sms / tail && s <= nkb && nkb < INT32_MAX / 2; ++s) {
         const int64_t kbs = (nkb + s - 1) / s, waves = (tail * s + sms - 1) / sms;
         if ((s - 1) * kbs >= nkb) continue;  // an empty last unit
@@ -1045,6 +1083,7 @@ void ozaki_setup(ContractionPlan &p) {
     const bool exact = p.form == MGB_FORM_OZAKI;
     int64_t units[2] = {0, 0};
     double us[2];
+    p.sum_kb = exact ? 0 : oz_sum_blocks(p);
     p.tile[0] = oz_tiling(p, false, units[0], us[0]);
     p.wide = false;
     if (exact && (p.adaptive || oz_wide(S))) {
@@ -1293,6 +1332,7 @@ static int ozaki_shape(const ContractionPlan &p, void *C, void *ws, bool split, 
     a.full = (int64_t)job.tiles_n * job.tiles_m * job.L;
     a.splits = 1;
     a.kbs = a.nkb;
+    a.fold = p.sum_kb / oz_chunk(3, false);
     if (split && tile.splits > 1) {
         a.full = tile.full;
         a.splits = tile.splits;
