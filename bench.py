@@ -630,10 +630,9 @@ def config2_bench(dev, steps=3):
                 # the permutation BackendBase stages: A(a,b,c,d,e) -> (b,d,a,c,e)
                 perm = ["b", "d", "a", "c", "e"]
                 Y = m.empty_colmajor([ext[i] for i in perm], tdt, dev)
-                modes = {lab: k for k, lab in enumerate(A.inds)}
+                modes = m.ops._modes_for(A.inds)
                 (xd, kx) = _lib.make_desc(*m.ops._desc_args(A.data, A.inds, modes))
-                (yd, ky) = _lib.make_desc(_lib.C64 if tdt == torch.complex128 else _lib.F64,
-                                          tuple(modes[m.Index(i)] for i in perm), tuple(Y.shape), tuple(Y.stride()))
+                (yd, ky) = _lib.make_desc(*m.ops._desc_args(Y, [m.Index(i) for i in perm], modes))
 
                 def perm_run():
                     _lib.check(lib.mgb_permute(ctypes.byref(xd), ctypes.byref(yd), A.data.data_ptr(), Y.data_ptr(),

@@ -17,7 +17,7 @@ import torch
 from . import _lib
 from ._lib import ArgumentError, check
 from .backend import Backend, DomainCUDA, choose_backend, register_rule
-from .tensor import Index, Tensor, empty_colmajor, intersect, nonunique, setdiff, union, unique
+from .tensor import Index, Tensor, empty_colmajor, intersect, nonunique, setdiff, union
 
 _DT = {torch.float32: _lib.F32, torch.float64: _lib.F64, torch.complex64: _lib.C32, torch.complex128: _lib.C64}
 _TORCH = {v: k for k, v in _DT.items()}
@@ -116,17 +116,21 @@ class _PlanCache:
 _PLANS = _PlanCache()
 
 
+def _key(i):
+    """What a label is compared by: an Index's tag (any other label is none's)."""
+    return i.tag if isinstance(i, Index) else (_key, i)
+
+
 def _modes_for(*label_lists) -> dict:
     m = {}
     for labels in label_lists:
         for i in labels:
-            if i not in m:
-                m[i] = len(m)
+            m.setdefault(i.tag if type(i) is Index else _key(i), len(m))
     return m
 
 
 def _desc_args(t: torch.Tensor, labels, modes: dict):
-    return (mgb_dtype(t.dtype), tuple(modes[i] for i in labels), tuple(t.shape), tuple(t.stride()))
+    return (mgb_dtype(t.dtype), tuple([modes[i.tag if type(i) is Index else _key(i)] for i in labels]), tuple(t.shape), tuple(t.stride()))
 
 
 def contraction_plan(a: torch.Tensor, ia, b: torch.Tensor, ib, c: torch.Tensor, ic, form: str = "auto",
@@ -217,13 +221,13 @@ class BackendGB300(Backend):
         inds_c = [i if isinstance(i, Index) else Index(i) for i in inds_c]
         sizes = {}
         for t in (a, b):
-            for d, i in enumerate(t.inds):
-                sizes.setdefault(i, t.data.shape[d])
+            for i, n in zip(t.inds, t.data.shape):
+                sizes.setdefault(i.tag, n)
         for i in inds_c:
-            if i not in sizes:
+            if i.tag not in sizes:
                 raise ArgumentError(f"output index {i} is in neither operand")
         dt = promote_eltype(a.dtype, b.dtype)
-        c = empty_colmajor([sizes[i] for i in inds_c], dt, a.data.device)
+        c = empty_colmajor([sizes[i.tag] for i in inds_c], dt, a.data.device)
         C = Tensor(c, inds_c)
         self.binary_einsum_(C, a, b)
         return C
@@ -236,8 +240,9 @@ class BackendGB300(Backend):
     # unary_einsum(::BackendGB300, inds_y, x)  (called at unary_einsum.jl:35)
     def unary_einsum(self, inds_y, x: Tensor) -> Tensor:
         inds_y = [i if isinstance(i, Index) else Index(i) for i in inds_y]
+        tags = [i.tag for i in x.inds]
         for i in inds_y:
-            if i not in x.inds:
+            if i.tag not in tags:
                 raise ArgumentError("Output indices must be a subset of input indices")
         y = empty_colmajor([x.size(i) for i in inds_y], x.dtype, x.data.device)
         Y = Tensor(y, inds_y)
@@ -275,7 +280,7 @@ class BackendGB300(Backend):
         _require_cuda(a.data, b.data, c.data)
         if list(c.inds) != list(a.inds):
             raise ArgumentError("hadamard!: inds(c) must equal inds(a)")
-        if any(i not in a.inds for i in b.inds):
+        if not _subset(b.inds, a.inds):
             raise ArgumentError("hadamard: inds(b) must be a subset of inds(a)")
         modes = _modes_for(a.inds)
         lib = _lib.load()
@@ -372,9 +377,24 @@ def binary_inds_c(ia, ib, dims=None, out=None) -> list:
     (src/Operations/binary_einsum.jl:33-40)."""
     if out is not None:
         return _labels(out)
-    dims = intersect(ia, ib) if dims is None else _labels(dims)
-    inds_sum = intersect(dims, ia, ib)
-    return setdiff(union(ia, ib), inds_sum)
+    if any(not isinstance(i, Index) for i in (*ia, *ib)):
+        dims = intersect(ia, ib) if dims is None else _labels(dims)
+        return setdiff(union(ia, ib), intersect(dims, ia, ib))
+    ta, tb = [i.tag for i in ia], [i.tag for i in ib]
+    td = ta if dims is None else [i.tag for i in _labels(dims)]
+    seen, inds_c = [], []
+    for i in (*ia, *ib):
+        t = i.tag
+        if t not in seen and not (t in ta and t in tb and t in td):
+            seen.append(t)
+            inds_c.append(i)
+    return inds_c
+
+
+def _subset(xs, ys) -> bool:
+    """Every label of xs is one of ys."""
+    tags = [y.tag for y in ys]
+    return all(x.tag in tags for x in xs)
 
 
 def unary_inds_y(ix, dims=None, out=None) -> list:
@@ -425,7 +445,7 @@ def hadamard(a: Tensor, b: Tensor) -> Tensor:
     must be a subset of the other's."""
     if a.ndim < b.ndim:
         a, b = b, a
-    if any(i not in a.inds for i in b.inds):
+    if not _subset(b.inds, a.inds):
         raise ArgumentError("hadamard: inds(b) must be a subset of inds(a)")
     backend = choose_backend(hadamard, a.data, b.data)
     return backend.hadamard(a, b)
@@ -438,7 +458,7 @@ def hadamard_(c: Tensor, a: Tensor, b: Tensor) -> Tensor:
         a, b = b, a
     if list(c.inds) != list(a.inds):
         raise ArgumentError("hadamard!: inds(c) must equal inds(a)")
-    if any(i not in a.inds for i in b.inds):
+    if not _subset(b.inds, a.inds):
         raise ArgumentError("hadamard!: inds(b) must be a subset of inds(a)")
     backend = choose_backend(hadamard_, c.data, a.data, b.data)
     backend.hadamard_(c, a, b)
@@ -447,9 +467,10 @@ def hadamard_(c: Tensor, a: Tensor, b: Tensor) -> Tensor:
 
 def _same_labels(xs, ys) -> bool:
     """The same labels, each as often, in any order."""
-    if len(xs) != len(ys) or any(x not in ys for x in xs):
-        return False
-    return len(unique(xs)) == len(xs) or sorted(map(repr, xs)) == sorted(map(repr, ys))
+    tx, ty = [x.tag for x in xs], [y.tag for y in ys]
+    if all(isinstance(t, str) for t in tx + ty):
+        return sorted(tx) == sorted(ty)
+    return sorted(map(repr, xs)) == sorted(map(repr, ys))
 
 
 def permutedims(t: Tensor, perm) -> Tensor:
@@ -457,13 +478,14 @@ def permutedims(t: Tensor, perm) -> Tensor:
     permutation kernel; ``perm`` is a list of Index labels or positions."""
     if t.ndim == 0:
         return t
-    labels = [t.inds[p] if isinstance(p, int) else (p if isinstance(p, Index) else Index(p)) for p in perm]
-    if not _same_labels(labels, t.inds):
+    inds = t.inds
+    labels = [inds[p] if isinstance(p, int) else (p if isinstance(p, Index) else Index(p)) for p in perm]
+    if not _same_labels(labels, inds):
         raise ArgumentError("permutation must use every label once")
     _require_cuda(t.data)
     y = empty_colmajor([t.size(i) for i in labels], t.dtype, t.data.device)
-    modes = _modes_for(t.inds)
-    (xd, kx) = _lib.kept_desc(*_desc_args(t.data, t.inds, modes))
+    modes = _modes_for(inds)
+    (xd, kx) = _lib.kept_desc(*_desc_args(t.data, inds, modes))
     (yd, ky) = _lib.kept_desc(*_desc_args(y, labels, modes))
     lib = _lib.load()
     check(lib.mgb_permute(ctypes.byref(xd), ctypes.byref(yd), t.data.data_ptr(), y.data_ptr(),

@@ -63,12 +63,12 @@ class Server:
         inds_c = binary_inds_c(a.inds, b.inds, dims, out)
         sizes = {}
         for t in (a, b):
-            for d, i in enumerate(t.inds):
-                sizes.setdefault(i, t.data.shape[d])
+            for i, n in zip(t.inds, t.data.shape):
+                sizes.setdefault(i.tag, n)
         for i in inds_c:
-            if i not in sizes:
+            if i.tag not in sizes:
                 raise ArgumentError(f"output index {i} is in neither operand")
-        c = empty_colmajor([sizes[i] for i in inds_c], promote_eltype(a.dtype, b.dtype), a.data.device)
+        c = empty_colmajor([sizes[i.tag] for i in inds_c], promote_eltype(a.dtype, b.dtype), a.data.device)
         C = Tensor(c, inds_c)
         plan = contraction_plan(a.data, a.inds, b.data, b.inds, c, inds_c, self.backend.form, self.backend.slices)
         resident = a.data.numel() * a.data.element_size() + b.data.numel() * b.data.element_size() + \
