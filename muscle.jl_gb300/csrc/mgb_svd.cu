@@ -20,6 +20,7 @@
 
 #include "mgb_internal.h"
 #include "mgb_ptx.h"
+#include "mgb_svd_wait.h"
 
 namespace mgb {
 
@@ -78,16 +79,17 @@ __device__ __forceinline__ uint32_t ld_acquire(const uint32_t *p) {
 __device__ __forceinline__ void st_release(uint32_t *p, uint32_t v) {
     asm volatile("st.release.gpu.global.u32 [%0], %1;" ::"l"(p), "r"(v) : "memory");
 }
-// Bounded wait for (*p & mask) >= v; false when it gave up (about a second of
+// Bounded wait for (*p & mask) >= v; false when it gave up (after `limit`
 // clock64 cycles) or another CTA did.
-__device__ __forceinline__ bool svd_wait(const uint32_t *p, uint32_t mask, uint32_t v, SvdSync *sy, int32_t *status) {
+__device__ __forceinline__ bool svd_wait(const uint32_t *p, uint32_t mask, uint32_t v, long long limit, SvdSync *sy,
+                                         int32_t *status) {
     if ((ld_acquire(p) & mask) >= v) return true;
     const long long t0 = clock64();
     for (uint32_t n = 1;; ++n) {
         if ((ld_acquire(p) & mask) >= v) return true;
         if ((n & 255) == 0) {
             if (ld_acquire(&sy->abort)) return false;
-            if (clock64() - t0 > kWaitTimeoutCycles) {
+            if (clock64() - t0 > limit) {
                 st_release(&sy->abort, 1u);
                 atomicCAS(status, 0, (int32_t)MGB_ERR_DEVICE_TIMEOUT);
                 return false;
@@ -286,6 +288,8 @@ __global__ void __launch_bounds__(kSvdThreads) k_svd_jacobi(T *__restrict__ W, i
     const int slot0 = cta * spc, slot1 = min(np, slot0 + spc);
     const int total = M + N;  // a column of W, then its column of V
     uint32_t done = 0;        // rounds completed, over all sweeps
+    const long long per_round = svd_wait_round(kWaitTimeoutCycles, M, N, spc);
+    const long long per_sweep = svd_wait_sweep(kWaitTimeoutCycles, M, N, spc, nct);
     auto pair = [&](int pi, int r, int &p, int &q) {
         p = circle(pi, r, nn);
         q = circle(nn - 1 - pi, r, nn);
@@ -301,8 +305,8 @@ __global__ void __launch_bounds__(kSvdThreads) k_svd_jacobi(T *__restrict__ W, i
         bool rotated = false;
         for (int r = 0; r + 1 < nn; ++r, ++done) {
             bool here = true;
-            if (tid == 0 && cta > 0) here = svd_wait(&sy->cta[cta - 1].rounds, ~0u, done, sy, status);
-            if (tid == 32 && cta + 1 < nct) here = svd_wait(&sy->cta[cta + 1].rounds, ~0u, done, sy, status);
+            if (tid == 0 && cta > 0) here = svd_wait(&sy->cta[cta - 1].rounds, ~0u, done, per_round, sy, status);
+            if (tid == 32 && cta + 1 < nct) here = svd_wait(&sy->cta[cta + 1].rounds, ~0u, done, per_round, sy, status);
             if (!__syncthreads_and(here)) {
                 ok = false;
                 break;
@@ -381,7 +385,7 @@ __global__ void __launch_bounds__(kSvdThreads) k_svd_jacobi(T *__restrict__ W, i
         if (!ok) break;
         if (tid == 0) {
             atomicAdd(&sy->sweep[sweep], rotated ? 0x10001u : 1u);
-            const bool met = svd_wait(&sy->sweep[sweep], 0xFFFFu, (uint32_t)nct, sy, status);
+            const bool met = svd_wait(&sy->sweep[sweep], 0xFFFFu, (uint32_t)nct, per_sweep, sy, status);
             agreed = met ? ld_acquire(&sy->sweep[sweep]) : 0u;  // final: every CTA has added its part
         }
         __syncthreads();
