@@ -49,8 +49,9 @@ struct Req {
     mgb_plan plan;
     const void *A, *B;
     void *C;
-    uint64_t ws;         // workspace bytes
-    uint64_t bytes;      // admitted bytes: caller-declared resident bytes + workspace
+    uint64_t ws;         // workspace bytes: the least the plan takes, or (started) what it asks for
+    uint64_t bytes;      // admitted bytes: caller-declared resident bytes + the least workspace
+    uint64_t extra = 0;  // workspace beyond it
     cudaEvent_t dep;     // caller-stream event the request waits on (or null)
     Clock::time_point t0;
     cudaEvent_t done = nullptr;    // the launch that computes it (set once known)
@@ -84,6 +85,8 @@ struct Batch {
 struct mgb_server_s {
     int device = 0;
     uint64_t budget = 0, used = 0;
+    uint64_t queued = 0;  // bytes of the pending requests
+    uint64_t extra = 0;   // part of `used`: room for split tiles
     int max_batch = 256;
     cudaMemPool_t pool = nullptr;
     std::vector<cudaStream_t> streams;
@@ -128,7 +131,8 @@ static void finish(mgb_server_s *s, const Req &r, int32_t status) {
     // caller holds s->mu
     s->finished[r.ticket] = status;
     s->latency_ms.push_back(std::chrono::duration<double, std::milli>(Clock::now() - r.t0).count());
-    s->used -= r.bytes;
+    s->used -= r.bytes + r.extra;
+    s->extra -= r.extra;
     ++s->completed;
     give_event(s, r.dep);
 }
@@ -344,8 +348,21 @@ static void serve_loop(mgb_server_s *s) {
                     Req &r = s->pending.front();
                     if (s->used + r.bytes > s->budget) break;  // wait for budget (FIFO)
                     s->used += r.bytes;
+                    s->queued -= r.bytes;
                     reqs.push_back(r);
                     s->pending.pop_front();
+                }
+                // Room for split tiles comes out of what the queue leaves free,
+                // and is a sixteenth of the budget at most, so that requests
+                // that come later find about as much as without it.
+                for (Req &r : reqs) {
+                    const uint64_t extra = r.plan->cp.ws_bytes - r.ws;
+                    if (extra && s->used + s->queued + extra <= s->budget && s->extra + extra <= s->budget / 16) {
+                        s->used += extra;
+                        s->extra += extra;
+                        r.extra = extra;
+                        r.ws += extra;
+                    }
                 }
             }
             if (reqs.empty()) break;
@@ -413,8 +430,7 @@ int mgb_server_submit(mgb_server server, mgb_plan plan, const void *A, const voi
     r.A = A;
     r.B = B;
     r.C = C;
-    // a request that the whole budget holds only without split tiles runs without them
-    r.ws = resident_bytes + plan->cp.ws_bytes <= server->budget ? plan->cp.ws_bytes : plan->cp.ws_min;
+    r.ws = plan->cp.ws_min;  // room for split tiles is added when it starts
     r.bytes = resident_bytes + r.ws;
     r.dep = nullptr;
     r.t0 = Clock::now();
@@ -433,6 +449,7 @@ int mgb_server_submit(mgb_server server, mgb_plan plan, const void *A, const voi
         r.dep = take_event(server);
         cudaEventRecord(r.dep, (cudaStream_t)dep_stream);
     }
+    server->queued += r.bytes;
     server->pending.push_back(r);
     server->cv_work.notify_one();
     return MGB_OK;
