@@ -1367,6 +1367,59 @@ static int ozaki_job(const ContractionPlan &p, void *C, void *ws, bool split, Oz
     return ozaki_maps(p, ws, S ? S : p.slices, false, &job.tmA, &job.tmB, job.band);
 }
 
+// The units of a launch of several jobs. Each job's cut is the best for it alone;
+// beside others that fill the GPU it mostly adds work: publishing a unit's sums
+// and adding them up takes 2.4 us: a burst of 600 served ComplexF64 requests of
+// one tile and 64 k blocks took 2945 us, each cut for itself, and takes 2384 so
+// (200 Float64 ones of 256 k blocks 2798, 2270). All cuts are thinned out by a
+// factor f = 1, 2, 4, .. (BF16X3: kept or dropped, its parts are fixed) to the
+// shortest launch, in k blocks per SM: the units and their overhead, and half of the
+// longest unit for the uneven end, but no less than that unit.
+static void ozaki_recut(std::vector<OzJob> &jobs, bool exact) {
+    if (jobs.size() < 2) return;
+    const double over = (OZ_SPLIT_FIXED + OZ_SPLIT_EACH) / oz_kb_us(exact, false), sms = sm_count();
+    struct Cut {
+        int32_t splits, kbs;
+    };
+    auto thin = [](const OzJob &j, int f) {
+        Cut c{1, j.a.nkb};
+        const int32_t s = (j.a.splits + f - 1) / f;
+        if (s > 1) {
+            c.kbs = f == 1 ? j.a.kbs : (j.a.nkb + s - 1) / s;
+            c.splits = (j.a.nkb + c.kbs - 1) / c.kbs;
+        }
+        return c;
+    };
+    int most = 1;
+    for (const OzJob &j : jobs) most = std::max(most, j.a.splits);
+    if (most == 1) return;
+    int best_f = 1;
+    double best = 0.0;
+    for (int f = 1;; f = exact ? 2 * f : most) {
+        double sum = 0.0, longest = 0.0;
+        for (const OzJob &j : jobs) {
+            const int64_t tiles = (int64_t)j.tiles_n * j.tiles_m * j.L;
+            const Cut c = thin(j, f);
+            sum += (double)tiles * j.a.nkb;
+            if (c.splits > 1) sum += over * (double)(tiles - j.a.full) * c.splits;
+            longest = std::max(longest, c.splits > 1 && j.a.full == 0 ? c.kbs + over : (double)j.a.nkb);
+        }
+        const double t = std::max(longest, sum / sms + 0.5 * longest);
+        if (f == 1 || t < best) {
+            best = t;
+            best_f = f;
+        }
+        if (f >= most) break;
+    }
+    if (best_f == 1) return;
+    for (OzJob &j : jobs) {
+        const Cut c = thin(j, best_f);
+        if (c.splits == 1) j.a.full = (int64_t)j.tiles_n * j.tiles_m * j.L;
+        j.a.splits = c.splits;
+        j.a.kbs = c.kbs;
+    }
+}
+
 // The job of every slice count in `cand`, of which `sel` (nullable) names the
 // one to run; without it cand is one count.
 static int ozaki_any_job(const ContractionPlan &p, void *C, void *ws, bool split, bool wide, uint32_t cand,
@@ -1477,8 +1530,9 @@ int ozaki_grouped_create(const std::vector<const ContractionPlan *> &plans, cons
             delete g;
             return st;
         }
-        start[i + 1] = start[i] + host[i].units();
     }
+    ozaki_recut(host, exact);
+    for (size_t i = 0; i < plans.size(); ++i) start[i + 1] = start[i] + host[i].units();
     g->njobs = (int)plans.size();
     g->tiles = start.back();
     cudaError_t e = cudaMalloc((void **)&g->jobs, host.size() * sizeof(OzJob));
@@ -1966,9 +2020,11 @@ int ozaki_batch_launch(const std::vector<OzBatchItem> &items, OzBatchBuffers *bu
     }
     // longest tiles first in every variant's launch: each CTA ends its walk
     // on short tiles, which even out the CTAs' finishing times
-    for (auto &kv : gem)
+    for (auto &kv : gem) {
+        ozaki_recut(kv.second, std::get<1>(kv.first) != 0);
         std::stable_sort(kv.second.begin(), kv.second.end(),
                          [](const OzJob &u, const OzJob &v) { return u.a.nkb > v.a.nkb; });
+    }
     // ---- one staging area: [pre-pass tables][per item: fixed slice count,
     //      address of its slice count][per variant: jobs, starts]
     auto al = al256;
