@@ -85,7 +85,7 @@ def union(*seqs) -> list:
 
 def empty_colmajor(shape: Sequence[int], dtype, device) -> torch.Tensor:
     """An uninitialised column-major (Julia-order) array."""
-    strides, acc = [], 1
+    shape, strides, acc = list(shape), [], 1
     for d in shape:
         strides.append(acc)
         acc *= max(d, 1)

@@ -5,9 +5,10 @@ import random
 
 import numpy as np
 import pytest
+import torch
 
 from muscle_gb300.ops import _desc_args, _modes_for, _same_labels, binary_inds_c
-from muscle_gb300.tensor import Index, Tensor, intersect, setdiff, union
+from muscle_gb300.tensor import Index, Tensor, empty_colmajor, intersect, setdiff, union
 
 
 def test_index_is_no_tuple():
@@ -48,3 +49,11 @@ def test_labels_that_are_no_index_stay_apart():
 def test_permutation_by_labels_of_another_type_is_refused(tags):
     assert _same_labels([Index(2), Index(1)], [Index(1), Index(2)])
     assert not _same_labels([Index(t) for t in tags], [Index(1), Index(2)]) or tags == ["1", "2"]
+
+
+def test_empty_colmajor_takes_any_iterable():
+    for shape in (iter([2, 0, 3]), (n for n in (2, 0, 3)), np.array([2, 0, 3])):
+        t = empty_colmajor(shape, torch.float64, "cpu")
+        assert tuple(t.shape) == (2, 0, 3) and t.stride() == (1, 2, 2)
+    with pytest.raises(RuntimeError):
+        empty_colmajor([2, -1], torch.float64, "cpu")
