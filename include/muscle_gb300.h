@@ -155,6 +155,12 @@ int mgb_plan_set_band(mgb_plan plan, int32_t band);
  * always; the result is the same contraction. Diagnostic only. No
  * counterpart in the reference. */
 int mgb_plan_operands_swapped(mgb_plan plan, int32_t *swapped);
+/* How the emulated GEMM of the plan runs: *wide is 1 in 128 x 64 tiles (an
+ * adaptive plan: with the slice counts that have them, 3 and 6), *splits[2]
+ * the units per tile that its last wave is cut into along K in narrow and in
+ * wide tiles (1: uncut; 0: not used). Diagnostic only. No counterpart in the
+ * reference. */
+int mgb_plan_tiling(mgb_plan plan, int32_t *wide, int32_t *splits);
 /* Target relative Frobenius error (> 0) of an adaptive plan's slice choice;
  * the default 1e-13 is the tolerance Muscle.jl's Float64 results are held
  * to. Set it before executing the plan, not while executions are in flight.

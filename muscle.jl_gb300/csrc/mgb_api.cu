@@ -396,6 +396,17 @@ int mgb_plan_operands_swapped(mgb_plan plan, int32_t *swapped) {
     return MGB_OK;
 }
 
+int mgb_plan_tiling(mgb_plan plan, int32_t *wide, int32_t *splits) {
+    if (!plan || !wide || !splits || plan->kind != PlanKind::Contraction)
+        return fail(MGB_ERR_ARGUMENT, "tiling: needs a contraction plan and outputs");
+    const ContractionPlan &cp = plan->cp;
+    const bool emulated = cp.form != MGB_FORM_PLAIN;
+    *wide = emulated && cp.wide ? 1 : 0;
+    splits[0] = emulated && (cp.adaptive || !cp.wide) ? cp.tile[0].splits : 0;
+    splits[1] = emulated && cp.wide ? cp.tile[1].splits : 0;
+    return MGB_OK;
+}
+
 int mgb_plan_set_band(mgb_plan plan, int32_t band) {
     if (!plan || plan->kind != PlanKind::Contraction) return fail(MGB_ERR_ARGUMENT, "band: not a contraction plan");
     if (band < 0 || band > 64) return fail(MGB_ERR_ARGUMENT, "band must be in 0..64");

@@ -68,6 +68,14 @@ class Plan:
         check(_lib.load().mgb_plan_operands_swapped(self.handle, ctypes.byref(v)))
         return bool(v.value)
 
+    @property
+    def tiling(self) -> dict:
+        """Whether the emulated GEMM runs in wide tiles, and the units that
+        the tiles of its last wave are cut into along K (narrow, wide)."""
+        wide, splits = ctypes.c_int32(0), (ctypes.c_int32 * 2)()
+        check(_lib.load().mgb_plan_tiling(self.handle, ctypes.byref(wide), splits))
+        return {"wide": bool(wide.value), "splits": tuple(splits)}
+
     def set_tolerance(self, tol: float) -> None:
         """Target relative Frobenius error of an adaptive plan's choice."""
         check(_lib.load().mgb_plan_set_tolerance(self.handle, float(tol)))
