@@ -53,6 +53,7 @@ struct Req {
     uint64_t bytes;      // admitted bytes: caller-declared resident bytes + the least workspace
     uint64_t extra = 0;  // workspace beyond it
     cudaEvent_t dep;     // caller-stream event the request waits on (or null)
+    bool dep_legacy;     // of the default stream
     Clock::time_point t0;
     cudaEvent_t done = nullptr;    // the launch that computes it (set once known)
     bool own_done = false;         // `done` belongs to this request alone
@@ -201,8 +202,13 @@ static int launch_emulated(mgb_server_s *s, size_t k) {
 static void launch_batch(mgb_server_s *s, size_t k, std::vector<Req> &reqs) {
     Batch &b = s->slots[k];
     cudaStream_t st = s->streams[k];
-    for (auto &r : reqs)
-        if (r.dep) cudaStreamWaitEvent(st, r.dep, 0);
+    // the last event of the default stream stands for those before it
+    bool legacy = false;
+    for (auto r = reqs.rbegin(); r != reqs.rend(); ++r) {
+        if (!r->dep || (r->dep_legacy && legacy)) continue;
+        cudaStreamWaitEvent(st, r->dep, 0);
+        legacy |= r->dep_legacy;
+    }
     std::vector<Req> failed;
     for (auto &r : reqs) (r.plan->cp.form == MGB_FORM_PLAIN ? b.plain : b.emu).push_back(r);
     if (!b.emu.empty()) {
@@ -433,6 +439,7 @@ int mgb_server_submit(mgb_server server, mgb_plan plan, const void *A, const voi
     r.ws = plan->cp.ws_min;  // room for split tiles is added when it starts
     r.bytes = resident_bytes + r.ws;
     r.dep = nullptr;
+    r.dep_legacy = (cudaStream_t)dep_stream == cudaStreamLegacy;
     r.t0 = Clock::now();
     std::lock_guard<std::mutex> lk(server->mu);
     r.ticket = server->next_ticket++;

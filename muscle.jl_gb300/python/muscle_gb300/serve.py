@@ -15,7 +15,7 @@ import torch
 
 from . import _lib
 from ._lib import ArgumentError, check
-from .ops import BackendGB300, binary_inds_c, contraction_plan, promote_eltype
+from .ops import BackendGB300, _stream_handle, binary_inds_c, contraction_plan, promote_eltype
 from .tensor import Index, Tensor, empty_colmajor
 
 
@@ -58,6 +58,12 @@ class Server:
         with torch.cuda.device(self.device):
             check(lib.mgb_server_create(ctypes.byref(self.handle), int(budget_bytes), int(streams), int(max_batch)), lib)
 
+    def _dependency(self) -> int:
+        """The current stream as a handle that is not null (the library takes a
+        null one as no dependency): the default stream goes by its other name,
+        cudaStreamLegacy."""
+        return _stream_handle(self.device) or 1
+
     def submit(self, a: Tensor, b: Tensor, dims=None, out=None, wait_for_stream: bool = True) -> Request:
         """Queues C = binary_einsum(a, b; dims, out); returns a Request."""
         inds_c = binary_inds_c(a.inds, b.inds, dims, out)
@@ -73,7 +79,7 @@ class Server:
         plan = contraction_plan(a.data, a.inds, b.data, b.inds, c, inds_c, self.backend.form, self.backend.slices)
         resident = a.data.numel() * a.data.element_size() + b.data.numel() * b.data.element_size() + \
             c.numel() * c.element_size()
-        dep = torch.cuda.current_stream(self.device).cuda_stream if wait_for_stream else None
+        dep = self._dependency() if wait_for_stream else None
         ticket = ctypes.c_int64(0)
         lib = _lib.load()
         check(lib.mgb_server_submit(self.handle, plan.handle, a.data.data_ptr(), b.data.data_ptr(), c.data_ptr(),
@@ -85,7 +91,7 @@ class Server:
         caller prepared (``contraction_plan`` on the same tensors)."""
         resident = a.data.numel() * a.data.element_size() + b.data.numel() * b.data.element_size() + \
             c.data.numel() * c.data.element_size()
-        dep = torch.cuda.current_stream(self.device).cuda_stream if wait_for_stream else None
+        dep = self._dependency() if wait_for_stream else None
         ticket = ctypes.c_int64(0)
         lib = _lib.load()
         check(lib.mgb_server_submit(self.handle, plan.handle, a.data.data_ptr(), b.data.data_ptr(),
