@@ -1321,7 +1321,7 @@ def main():
                     "result_matches_device_run": e2e_ok, "phases": e2e_phases},
             "roofline": {"bound": "tensor", "achieved": achieved, "peak": bf16_peak, "unit": "TFLOP/s",
                          "frac": achieved / bf16_peak, "traffic": traffic, "peak_kind": f"bf16 dense burst ({peak_kind})",
-                         "kernel": "k_oz_gemm_wide" if S in (3, 6) else "k_oz_gemm_any", "kernel_ms": gemm_ms, "prepass_ms": prepass_ms,
+                         "kernel": "k_oz_gemm_wide" if plan.tiling["wide"] and S in (3, 6) else "k_oz_gemm_any", "kernel_ms": gemm_ms, "prepass_ms": prepass_ms,
                          "prepass_bytes": prepass_bytes, "prepass_gbs": prepass_bytes / (prepass_ms / 1e3) / 1e9,
                          "prepass_frac_of_hbm": prepass_bytes / (prepass_ms / 1e3) / 1e9 / hbm_peak,
                          "work": f"2 x {pairs} slice pairs x M x 2N x 2K bf16 flops per launch"},

@@ -252,10 +252,12 @@ int mgb_group_destroy(mgb_group group);
  * later arrivals are admitted as budget frees up and launched on the other
  * streams, so their work overlaps on the GPU. A request's admitted bytes are
  * the caller-declared resident bytes (operands and output, which stay in
- * device memory owned by the caller) plus its workspace, which the server
- * allocates from its own stream-ordered pool. A request larger than the
- * whole budget finishes at once with MGB_ERR_OUT_OF_MEMORY. `dep_stream`
- * (may be NULL) is a caller stream whose work so far the request waits for
+ * device memory owned by the caller) plus the least workspace its plan runs
+ * with, which the server allocates from its own stream-ordered pool; up to a
+ * sixteenth of the budget goes to requests that run faster with more. A
+ * request larger than the whole budget finishes at once with
+ * MGB_ERR_OUT_OF_MEMORY. `dep_stream` (NULL: none; cudaStreamLegacy: the
+ * default stream) is a caller stream whose work so far the request waits for
  * (e.g. the kernels that produced its operands). Plans and buffers must stay
  * alive until mgb_server_wait has returned for the ticket. This is the
  * request loop of the serving form; the reference has no counterpart.     */
@@ -318,10 +320,11 @@ int mgb_selftest_wait_timeout(void *stream);
  * s to unit 2-norm (normalize! of simple_update); MGB_SVD_CONJ_V writes
  * conj(V), the right factor as tensor_svd_thin labels it; MGB_SVD_SQRT_S
  * writes sqrt of the (normalised) s, for an equal absorb. One-sided Jacobi
- * rotations on the device, a pair of columns per SM in one cooperative
- * launch: min(m, n) <= 1024, m n <= 2^28. Left vectors of exactly zero
- * singular values are completed to an orthonormal set. The workspace comes
- * from mgb_svd_workspace_size.                                            */
+ * rotations on the device, in one thread-block cluster (max(m, n) <= 256,
+ * min(m, n) <= 128) or one cooperative launch: min(m, n) <= 1024, m n <=
+ * 2^28. Squares of the entries should lie in the range of doubles. Left
+ * vectors of exactly zero singular values are completed to an orthonormal
+ * set. The workspace comes from mgb_svd_workspace_size.                   */
 #define MGB_SVD_NORMALIZE 1
 #define MGB_SVD_CONJ_V 2
 #define MGB_SVD_SQRT_S 4

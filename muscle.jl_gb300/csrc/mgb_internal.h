@@ -147,7 +147,7 @@ struct ContractionPlan {
     uint64_t ws_cnt = 0, ws_part = 0;  // counters and sums of split tiles
     OzTiling tile[2];   // narrow and wide tiles of the emulated GEMM
     int32_t sum_kb = 0; // BF16X3: k blocks per partial sum of every tile (0: one sum)
-    bool wide = false;  // run in wide tiles where the slice count has them (not in a group)
+    bool wide = false;  // run in wide tiles where the slice count has them (not from a job table)
     uint64_t ws_a = 0, ws_b = 0, ws_scale_a = 0, ws_scale_b = 0;
     int64_t kpad = 0;      // padded embedded K of the slice buffers
     int64_t m_e = 0, n_e = 0, k_e = 0;  // embedded GEMM extents
@@ -197,8 +197,8 @@ int selftest_wait_timeout(cudaStream_t s);
 // slices, form and real/complex) whose slices lie in the given workspaces.
 int ozaki_prepass(const ContractionPlan &p, const void *A, const void *B, void *ws, bool split, cudaStream_t s);
 // The tensor-core part of one plan whose pre-pass has run into `ws` (for an
-// adaptive plan: one launch per candidate slice count, of which only the
-// chosen one works, and the plain form as the fallback).
+// adaptive plan: one launch that reads the chosen slice count, or one for the
+// counts of wide tiles and one for the others, and the plain form as the fallback).
 int ozaki_gemm(const ContractionPlan &p, const void *A, const void *B, void *C, void *ws, bool split, cudaStream_t s);
 // Reads the adaptive choice of the last call that ran with `ws` (synchronises s).
 int ozaki_adaptive_report(const ContractionPlan &p, const void *ws, cudaStream_t s, mgb_adaptive_report *out);

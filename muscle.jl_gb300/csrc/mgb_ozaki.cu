@@ -1631,7 +1631,6 @@ __global__ void __launch_bounds__(256) k_oz_pre_multi(const PreJob *__restrict__
     oz_stat_block(J.part, J.exps, J.st, J.t, J.q, J.P, J.g.R, J.g.K, blk, l, sm);
 }
 
-// dst[i] = *src[i]: every item's slice count after the choice
 // The last job of a table whose first block is <= b.
 __device__ __forceinline__ int multi_job(const int64_t *__restrict__ start, int njobs, int64_t b) {
     int lo = 0, hi = njobs - 1;
@@ -1678,12 +1677,12 @@ __global__ void __launch_bounds__(256, OZ_SLICE_OCC) k_oz_slice_multi(const PreJ
     oz_slice_tile<T, MODE, BF3>((const T *)J.X, J.g, J.exps, S, J.out, J.rows_e, J.kw, local - l * per_l, l, sm);
 }
 
+// dst[i] = *src[i]: every item's slice count after the choice
 __global__ void k_gather_sel(const int32_t *const *__restrict__ src, int32_t *__restrict__ dst, int n) {
     const int i = blockIdx.x * blockDim.x + threadIdx.x;
     if (i < n) dst[i] = *src[i];
 }
 
-// One block per adaptive contraction (the body of k_oz_choose).
 // The estimate's sums of every adaptive contraction of a batch: job j owns
 // blocks [start[j], start[j + 1]) (oz_est_blocks(K) per batch entry).
 __global__ void __launch_bounds__(256) k_oz_est_multi(const ChooseJob *__restrict__ jobs,
