@@ -199,13 +199,19 @@ def contract_into(c: torch.Tensor, ic, a: torch.Tensor, ia, b: torch.Tensor, ib,
     _require_cuda(a, b, c)
     plan = contraction_plan(a, ia, b, ib, c, ic, form, slices)
     need = plan.workspace_bytes
+    lib = _lib.load()
+    stream = _stream_handle(c.device)
     if workspace is not None and workspace.numel() >= need:
         ws, wp = workspace, workspace.data_ptr()
     else:
+        if workspace is not None:  # it may still be enough to run without split tiles
+            st = lib.mgb_contract(plan.handle, a.data_ptr(), b.data_ptr(), c.data_ptr(), workspace.data_ptr(),
+                                  workspace.numel(), stream)
+            if st != _lib.ERR_WORKSPACE:
+                check(st, lib)
+                return c
         ws, wp = _workspace(need, c.device)
-    lib = _lib.load()
-    check(lib.mgb_contract(plan.handle, a.data_ptr(), b.data_ptr(), c.data_ptr(), wp, need,
-                           _stream_handle(c.device)), lib)
+    check(lib.mgb_contract(plan.handle, a.data_ptr(), b.data_ptr(), c.data_ptr(), wp, need, stream), lib)
     return c
 
 
