@@ -222,12 +222,12 @@ struct OzGemmArgs {
     // units leave their sums in `part` and count in `cnt` (zero before and
     // after); the last one adds them up and writes the outputs.
     int32_t splits, kbs;
-    // BF16X3: chunks per partial sum of a whole tile (0: one sum), those of the
-    // units that it would be cut into (see oz_sum_blocks)
-    int32_t fold;
     int64_t full;
     uint32_t *part;
     int32_t *cnt;
+    // BF16X3: chunks per partial sum of a whole tile (0: one sum), those of the
+    // units that it would be cut into (see oz_sum_blocks)
+    int32_t fold;
 };
 
 // One contraction (or one bucket of a group) as the GEMM sees it: the slice
@@ -405,19 +405,16 @@ __device__ __forceinline__ uint4 *oz_part_at(uint32_t *part, int unit, int w) {
     return (uint4 *)part + (((int64_t)unit * OZ_EPI_WARPS + w) * (NW / 4)) * 32 + threadIdx.x % 32;
 }
 // Publishes this warp's share and counts it; true for the warp that finds all
-// `splits` shares of its tile published, which sets the counter back to zero:
+// `splits` shares of its tile published, whose count wraps to zero:
 // the GEMM may run again on the same slices. Nobody waits for anybody.
 __device__ __forceinline__ bool oz_part_last(int32_t *cnt, int tile, int w, int splits) {
     __threadfence();
     __syncwarp();
-    int old = 0;
-    int32_t *c = cnt + tile * OZ_EPI_WARPS + w;
-    if (threadIdx.x % 32 == 0) old = atomicAdd(c, 1);
-    const bool last = __shfl_sync(0xffffffffu, old, 0) == splits - 1;
-    if (last) {
-        if (threadIdx.x % 32 == 0) *c = 0;
-        __threadfence();
-    }
+    uint32_t old = 0;
+    if (threadIdx.x % 32 == 0)  // the last increment wraps to zero
+        old = atomicInc((uint32_t *)cnt + tile * OZ_EPI_WARPS + w, (uint32_t)splits - 1);
+    const bool last = __shfl_sync(0xffffffffu, old, 0) == (uint32_t)splits - 1;
+    if (last) __threadfence();
     return last;
 }
 
