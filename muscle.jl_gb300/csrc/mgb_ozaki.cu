@@ -976,7 +976,7 @@ constexpr int64_t OZ_SUM_SMS = 152;
 static int32_t oz_sum_blocks(const ContractionPlan &p) {
     const int64_t bn = oz_bn(3, false), chunk = oz_chunk(3, false);
     const int64_t tiles = ((p.m_e + OZ_BM - 1) / OZ_BM) * ((p.n_e + bn - 1) / bn), nkb = (p.k_e + OZ_BK - 1) / OZ_BK;
-    if (tiles == 0 || tiles >= OZ_SUM_SMS || nkb >= INT32_MAX / 2) return 0;
+    if (tiles == 0 || tiles >= OZ_SUM_SMS || nkb <= chunk || nkb >= INT32_MAX / 2) return 0;
     const double kb = oz_kb_us(false, false);
     double best = nkb * kb - OZ_SPLIT_GAIN;
     int64_t kbs = 0;
