@@ -138,7 +138,8 @@ def _modes_for(*label_lists) -> dict:
 
 
 def _desc_args(t: torch.Tensor, labels, modes: dict):
-    return (mgb_dtype(t.dtype), tuple([modes[i.tag if type(i) is Index else _key(i)] for i in labels]), tuple(t.shape), tuple(t.stride()))
+    m = tuple([modes[i.tag if type(i) is Index else _key(i)] for i in labels])
+    return (mgb_dtype(t.dtype), m, tuple(t.shape), tuple(t.stride()))
 
 
 def contraction_plan(a: torch.Tensor, ia, b: torch.Tensor, ib, c: torch.Tensor, ic, form: str = "auto",
